@@ -19,6 +19,7 @@ namespace nsfv1 {
 
 static constexpr int kRedBlocks = 608;   // 4 x 152 SMs
 static constexpr int kRedThreads = 256;
+static constexpr int kGmresScal = 256;   // the GMRES state follows the first 256 scalars of Workspace::scal
 
 // ---------------------------------------------------------------------------
 // block SpMV y = A x: one group of G lanes per block row; lane l takes the
@@ -619,65 +620,386 @@ __global__ void k_set_dirichlet(int64_t n, const int32_t* __restrict__ rows, con
     if (i < n) u[rows[i]] = vals[i];
 }
 
-// GMRES helpers ---------------------------------------------------------------
-// h[k] = (V_k, w) for k < m (one pass over w, partials per block)
-template <typename VT>
-__global__ void __launch_bounds__(kRedThreads) k_multidot_partial(int64_t n, int m, const VT* __restrict__ V, const VT* __restrict__ w,
-                                                                 double* __restrict__ partials) {
-    __shared__ double sh[kRedThreads];
-    for (int k = 0; k < m; ++k) {
-        double acc = 0.0;
-        const VT* vk = V + (int64_t)k * n;
-        for (int64_t i = (int64_t)blockIdx.x * kRedThreads + threadIdx.x; i < n; i += (int64_t)gridDim.x * kRedThreads)
-            acc += (double)vk[i] * (double)w[i];
-        sh[threadIdx.x] = acc;
-        __syncthreads();
-        for (int s = kRedThreads / 2; s > 0; s >>= 1) {
-            if (threadIdx.x < s) sh[threadIdx.x] += sh[threadIdx.x + s];
-            __syncthreads();
+// GMRES -----------------------------------------------------------------------
+// One iteration is five launches and no host read: the scalar work (Gram-Schmidt
+// sums, Givens rotations, stop tests) is done by the last block of each reduction.
+// Four FP64 multiply-adds per basis entry on a pipe that takes a warp instruction
+// every 19 clocks per SM (about 14 us an iteration at 192^2 quadrilaterals, n =
+// 111,747, 16 basis vectors) and the L2 round trips of the reductions bound it:
+// 68 us an iteration there (GMRES(30), 45 iterations in 3.04 ms; 64^2: 44 us). With
+// one dot product per pass over w, a single-block sum of every coefficient and three
+// host reads an iteration it was 214 us (9.64 ms; 64^2: 200 us). Launching the five
+// kernels with programmatic stream serialisation measured the same (3.12 ms).
+// Scalars in device memory at Workspace::scal + kGmresScal:
+enum { G_DONE = 0, G_J, G_IT, G_RELRES, G_BETA0, G_INV, G_HN, G_H1 = 8, G_H2 = G_H1 + 66, G_CS = G_H2 + 66, G_SN = G_CS + 64,
+       G_GAM = G_SN + 64, G_Y = G_GAM + 66, G_HES = G_Y + 64, G_NSCAL = G_HES + 65 * 64 };
+// G_DONE: 0 iterating, 1 the cycle ends (converged or hn = 0), 2 non-finite
+enum { GM_CYCLE_END = 1, GM_NONFINITE = 2 };
+
+static constexpr int kGmT = 256;                     // threads, and entries of a tile
+static constexpr int kGmWarps = kGmT / 32;
+static constexpr int kGmBlocks = 2 * 152;            // the last block sums this many partials per coefficient
+static constexpr int kGmMaxM = 64;
+static constexpr int kGmPerWarp = (kGmMaxM + 1 + kGmWarps - 1) / kGmWarps;
+
+// Warp sums of four values with 6 additions instead of 20 (an FP64 instruction of a warp holds
+// the pipe for 16 clocks whatever its active lanes): the halves of the warp first split the
+// values between them. A lane ends with the sum of v[gm_owned(lane)].
+__device__ __forceinline__ double gm_warp_sum4(const double (&v)[4], const int lane) {
+    const bool up = lane & 16, uq = lane & 8;
+    double a = (up ? v[2] : v[0]) + __shfl_xor_sync(0xffffffffu, up ? v[0] : v[2], 16);
+    double c = (up ? v[3] : v[1]) + __shfl_xor_sync(0xffffffffu, up ? v[1] : v[3], 16);
+    double r = (uq ? c : a) + __shfl_xor_sync(0xffffffffu, uq ? a : c, 8);
+#pragma unroll
+    for (int off = 4; off > 0; off >>= 1) r += __shfl_xor_sync(0xffffffffu, r, off);
+    return r;
+}
+__device__ __forceinline__ int gm_owned(const int lane) { return ((lane & 16) >> 3) | ((lane & 8) >> 3); }
+
+// Each warp holds the partial sums acc[q] of coefficients warp + q * kGmWarps <= j; they
+// go to partials[k * gridDim.x + block], and the block that finishes last sums them over the
+// blocks in a fixed order into h[0..j] and returns true (all threads; h visible to them).
+__device__ __forceinline__ bool gm_reduce(const double (&acc)[kGmPerWarp], const int j, double* __restrict__ partials, unsigned* counter,
+                                          double* h) {
+    __shared__ bool amLast;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nb = gridDim.x;
+    const int mine = gm_owned(lane);
+#pragma unroll
+    for (int q0 = 0; q0 < kGmPerWarp; q0 += 4) {
+        if (warp + q0 * kGmWarps > j) break;
+        double v[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = q0 + i < kGmPerWarp ? acc[q0 + i < kGmPerWarp ? q0 + i : 0] : 0.0;
+        const double r = gm_warp_sum4(v, lane);
+        const int k = warp + (q0 + mine) * kGmWarps;
+        if ((lane & 7) == 0 && k <= j) partials[k * nb + blockIdx.x] = r;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        amLast = atomicAdd(counter, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!amLast) return false;
+    __threadfence();
+    constexpr int U = (kGmBlocks + 31) / 32;
+    for (int k0 = warp; k0 <= j; k0 += 4 * kGmWarps) {
+        // every load of the four sums is issued before the first addition
+        double pv[4][U];
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int i = 0; i < U; ++i) {
+                const int k = k0 + c * kGmWarps, q = lane + 32 * i;
+                pv[c][i] = k <= j && q < nb ? __ldcg(partials + k * nb + q) : 0.0;
+            }
+        double v[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            if (k0 + c * kGmWarps > j) break;
+#pragma unroll
+            for (int i = 0; i < U; ++i)
+                if (32 * i < nb) v[c] += pv[c][i];
         }
-        if (threadIdx.x == 0) partials[k * gridDim.x + blockIdx.x] = sh[0];
+        const double r = gm_warp_sum4(v, lane);
+        const int k = k0 + mine * kGmWarps;
+        if ((lane & 7) == 0 && k <= j) h[k] = r;
+    }
+    if (threadIdx.x == 0) *counter = 0u;
+    __syncthreads();
+    return true;
+}
+
+// the block sum of v over the grid (the last block; valid in its thread 0), as gm_reduce
+__device__ __forceinline__ bool gm_reduce1(double v, double* __restrict__ partials, unsigned* counter, double& out) {
+    __shared__ bool amLast;
+    __shared__ double sh[kGmWarps];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nb = gridDim.x;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+    if (lane == 0) sh[warp] = v;
+    __syncthreads();
+    if (warp == 0) {
+        double a = sh[lane & (kGmWarps - 1)];
+#pragma unroll
+        for (int off = kGmWarps / 2; off > 0; off >>= 1) a += __shfl_xor_sync(0xffffffffu, a, off);
+        if (lane == 0) {
+            partials[blockIdx.x] = a;
+            __threadfence();
+            amLast = atomicAdd(counter, 1u) == gridDim.x - 1;
+        }
+    }
+    __syncthreads();
+    if (!amLast) return false;
+    __threadfence();
+    v = 0.0;
+    for (int i = threadIdx.x; i < nb; i += kGmT) v += __ldcg(partials + i);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+    if (lane == 0) sh[warp] = v;
+    __syncthreads();
+    if (warp == 0) {
+        out = sh[lane & (kGmWarps - 1)];
+#pragma unroll
+        for (int off = kGmWarps / 2; off > 0; off >>= 1) out += __shfl_xor_sync(0xffffffffu, out, off);
+        if (lane == 0) *counter = 0u;
+    }
+    return true;
+}
+
+// the entries of this block: an even split of n over the grid in whole warps
+__device__ __forceinline__ void gm_range(const int64_t n, int64_t& i0, int64_t& i1) {
+    const int64_t per = ((n + gridDim.x - 1) / gridDim.x + 31) / 32 * 32;
+    i0 = min(n, per * blockIdx.x);
+    i1 = min(n, i0 + per);
+}
+
+// start of a cycle: V_0 = rhs - J x (w = J x, or null for x = 0) and its norm; the last block
+// sets the stop state (converged at the start of a cycle, zero right-hand side) and 1 / beta
+__global__ void __launch_bounds__(kGmT) k_gm_start(int64_t n, const double* __restrict__ rhs, const double* __restrict__ w, double* __restrict__ V0,
+                                                   double* __restrict__ partials, unsigned* counter, double* G, double rtol) {
+    double acc = 0.0;
+    int64_t i0, i1;
+    gm_range(n, i0, i1);
+    for (int64_t i = i0 + threadIdx.x; i < i1; i += kGmT) {
+        const double v = w ? rhs[i] - w[i] : rhs[i];
+        V0[i] = v;
+        acc += v * v;
+    }
+    double s;
+    if (!gm_reduce1(acc, partials, counter, s) || threadIdx.x != 0) return;
+    const double beta = sqrt(s);
+    if (!w) G[G_BETA0] = beta;
+    const double beta0 = G[G_BETA0];
+    G[G_RELRES] = beta0 == 0.0 ? 1.0 : beta / beta0;
+    G[G_J] = 0.0;
+    G[G_INV] = 1.0 / beta;
+    G[G_GAM] = beta;
+    // beta = 0, or below the tolerance: nothing to iterate (the host leaves the loop)
+    G[G_DONE] = (beta0 == 0.0 || G[G_RELRES] < rtol) ? GM_CYCLE_END : 0.0;
+}
+
+// h1[k] = (V_k, w), k <= j: a tile of w goes to shared memory, each warp streams the tiles of
+// its own basis vectors
+__global__ void __launch_bounds__(kGmT) k_gm_dots(int64_t n, int j, const double* __restrict__ V, const double* __restrict__ w,
+                                                  double* __restrict__ partials, unsigned* counter, double* G) {
+    if (G[G_DONE] != 0.0) return;
+    __shared__ double sw[kGmT];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double acc[kGmPerWarp];
+#pragma unroll
+    for (int q = 0; q < kGmPerWarp; ++q) acc[q] = 0.0;
+    int64_t i0, i1;
+    gm_range(n, i0, i1);
+    for (int64_t t0 = i0; t0 < i1; t0 += kGmT) {
+        const int cnt = (int)min((int64_t)kGmT, i1 - t0);
+        __syncthreads();
+        sw[threadIdx.x] = threadIdx.x < cnt ? w[t0 + threadIdx.x] : 0.0;
+        __syncthreads();
+#pragma unroll
+        for (int q0 = 0; q0 < kGmPerWarp; q0 += 4) {
+            if (warp + q0 * kGmWarps > j) break;
+            // the loads of four basis vectors are issued before the first product
+            double v[4][kGmT / 32];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const int k = warp + (q0 + c) * kGmWarps;
+                const double* vk = V + (int64_t)k * n + t0;
+#pragma unroll
+                for (int i = 0; i < kGmT / 32; ++i) v[c][i] = k <= j && lane + 32 * i < cnt ? vk[lane + 32 * i] : 0.0;
+            }
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                if (q0 + c >= kGmPerWarp || warp + (q0 + c) * kGmWarps > j) break;
+#pragma unroll
+                for (int i = 0; i < kGmT / 32; ++i)
+                    if (32 * i < cnt) acc[q0 + c < kGmPerWarp ? q0 + c : 0] += v[c][i] * sw[lane + 32 * i];
+            }
+        }
+    }
+    gm_reduce(acc, j, partials, counter, G + G_H1);
+}
+
+// w -= sum_k h1[k] V_k and h2[k] = (V_k, w) of the result: one pass over the basis, whose tile
+// stays in shared memory between the two
+__global__ void __launch_bounds__(kGmT) k_gm_axpy_dots(int64_t n, int j, const double* __restrict__ V, double* __restrict__ w,
+                                                       double* __restrict__ partials, unsigned* counter, double* G) {
+    if (G[G_DONE] != 0.0) return;
+    extern __shared__ double sv[];   // [j + 1][kGmT] basis tile, then [kGmT] w
+    __shared__ double sh[kGmMaxM + 1];
+    double* sw = sv + (j + 1) * kGmT;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = threadIdx.x;
+    if (t <= j) sh[t] = G[G_H1 + t];
+    __syncthreads();
+    double acc[kGmPerWarp];
+#pragma unroll
+    for (int q = 0; q < kGmPerWarp; ++q) acc[q] = 0.0;
+    int64_t i0, i1;
+    gm_range(n, i0, i1);
+    for (int64_t t0 = i0; t0 < i1; t0 += kGmT) {
+        const int cnt = (int)min((int64_t)kGmT, i1 - t0);
+        if (32 * warp < cnt) {
+            const bool in = t < cnt;
+            double a = in ? w[t0 + t] : 0.0;
+            // asynchronous copies keep the whole tile in flight; a thread reads back only its own entries here
+            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(sv + t);
+            const double* v0 = V + t0 + (in ? t : 0);
+            for (int k = 0; k <= j; ++k)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst + k * (kGmT * 8)), "l"(v0 + (int64_t)k * n), "r"(in ? 8 : 0)
+                             : "memory");
+            asm volatile("cp.async.wait_all;" ::: "memory");
+#pragma unroll 4
+            for (int k = 0; k <= j; ++k) a -= sh[k] * sv[k * kGmT + t];
+            sw[t] = a;
+            if (in) w[t0 + t] = a;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < kGmPerWarp; ++q) {
+            const int k = warp + q * kGmWarps;
+            if (k > j) break;
+#pragma unroll
+            for (int i = 0; i < kGmT / 32; ++i)
+                if (32 * i < cnt) acc[q] += sv[k * kGmT + lane + 32 * i] * sw[lane + 32 * i];
+        }
         __syncthreads();
     }
+    gm_reduce(acc, j, partials, counter, G + G_H2);
 }
-__global__ void k_multidot_final(const double* __restrict__ partials, int nb, int m, double* out) {
-    __shared__ double sh[kRedThreads];
-    for (int k = 0; k < m; ++k) {
-        double acc = 0.0;
-        for (int i = threadIdx.x; i < nb; i += kRedThreads) acc += partials[k * nb + i];
-        sh[threadIdx.x] = acc;
-        __syncthreads();
-        for (int s = kRedThreads / 2; s > 0; s >>= 1) {
-            if (threadIdx.x < s) sh[threadIdx.x] += sh[threadIdx.x + s];
-            __syncthreads();
+
+// w -= sum_k h2[k] V_k and its norm hn; the last block stores hn and 1 / hn
+__global__ void __launch_bounds__(kGmT) k_gm_end(int64_t n, int j, const double* __restrict__ V, double* __restrict__ w,
+                                                 double* __restrict__ partials, unsigned* counter, double* G) {
+    if (G[G_DONE] != 0.0) return;
+    __shared__ double sh[kGmMaxM + 1];
+    if (threadIdx.x <= j) sh[threadIdx.x] = G[G_H2 + threadIdx.x];
+    __syncthreads();
+    double acc = 0.0;
+    int64_t i0, i1;
+    gm_range(n, i0, i1);
+    for (int64_t i = i0 + threadIdx.x; i < i1; i += kGmT) {
+        double a = w[i];
+        for (int k0 = 0; k0 <= j; k0 += 16) {
+            // sixteen loads in flight
+            double v[16];
+#pragma unroll
+            for (int c = 0; c < 16; ++c) v[c] = k0 + c <= j ? V[(int64_t)(k0 + c) * n + i] : 0.0;
+#pragma unroll
+            for (int c = 0; c < 16; ++c) {
+                if (k0 + c > j) break;
+                a -= sh[k0 + c] * v[c];
+            }
         }
-        if (threadIdx.x == 0) out[k] = sh[0];
-        __syncthreads();
+        w[i] = a;
+        acc += a * a;
+    }
+    double s;
+    if (!gm_reduce1(acc, partials, counter, s) || threadIdx.x != 0) return;
+    const double hn = sqrt(s);
+    G[G_HN] = hn;
+    G[G_INV] = 1.0 / hn;
+    G[G_J] = j + 1;   // columns whose basis vectors exist
+}
+
+// the scalar end of iteration j (one block): the Hessenberg column h1 + h2, the Givens
+// rotations, the residual estimate and the stop tests. The rotations are one serial chain of
+// FP64 operations (64 clocks each): its inputs come to shared memory first.
+__device__ __forceinline__ void gm_givens(double* G, const int j, const int m, const double rtol) {
+    __shared__ double hc[kGmMaxM + 1], cs[kGmMaxM], sn[kGmMaxM];
+    const int t = threadIdx.x;
+    if (t <= j) hc[t] = G[G_H1 + t] + G[G_H2 + t];
+    if (t < j) { cs[t] = G[G_CS + t]; sn[t] = G[G_SN + t]; }
+    __syncthreads();
+    if (t == 0) {
+        const double hn = G[G_HN], gj = G[G_GAM + j], beta0 = G[G_BETA0], it = G[G_IT];
+        double hk = hc[0];
+        for (int k = 0; k < j; ++k) {
+            const double nx = hc[k + 1];
+            hc[k] = cs[k] * hk + sn[k] * nx;
+            hk = -sn[k] * hk + cs[k] * nx;
+        }
+        const double rr = sqrt(hk * hk + hn * hn);
+        const double c = rr > 0.0 ? hk / rr : 1.0, sj = rr > 0.0 ? hn / rr : 0.0;
+        hc[j] = rr;
+        G[G_CS + j] = c;
+        G[G_SN + j] = sj;
+        G[G_GAM + j + 1] = -sj * gj;
+        G[G_GAM + j] = c * gj;
+        const double relres = fabs(sj * gj) / beta0;
+        G[G_RELRES] = relres;
+        G[G_IT] = it + 1.0;
+        if (!isfinite(relres)) G[G_DONE] = GM_NONFINITE;
+        else if (relres < rtol || hn == 0.0) G[G_DONE] = GM_CYCLE_END;
+    }
+    __syncthreads();
+    if (t <= j) G[G_HES + t * m + j] = hc[t];   // H[k * m + column]
+}
+
+__global__ void __launch_bounds__(kGmT) k_gm_givens(double* G, int j, int m, double rtol) {
+    if (G[G_DONE] == 0.0) gm_givens(G, j, m, rtol);
+}
+
+// V_j *= 1 / norm; Z_j = Dinv V_j (the point-block Jacobi apply of k_prec, same summation).
+// The last block ends iteration j - 1 (gm_givens) meanwhile: up to 5 us of serial FP64 that
+// would otherwise stand at the tail of k_gm_end. A stop found there lets this kernel's writes
+// stand (V_j and Z_j are not used after a stop).
+template <typename MT, int b>
+__global__ void __launch_bounds__(kGmT) k_gm_prec(int64_t nRows, double* G, double* __restrict__ Vj, const MT* __restrict__ Dinv,
+                                                  double* __restrict__ Zj, int j, int m, double rtol) {
+    if (blockIdx.x == gridDim.x - 1) {
+        if (j > 0 && G[G_DONE] == 0.0) gm_givens(G, j - 1, m, rtol);
+        return;
+    }
+    const int64_t r = (int64_t)blockIdx.x * kGmT + threadIdx.x;
+    if (r >= nRows) return;
+    const double inv = G[G_INV];
+    double x[b];
+#pragma unroll
+    for (int i = 0; i < b; ++i) {
+        x[i] = Vj[r * b + i] * inv;
+        Vj[r * b + i] = x[i];
+    }
+    const MT* M = Dinv + r * b * b;
+#pragma unroll
+    for (int i = 0; i < b; ++i) {
+        double a = 0.0;
+#pragma unroll
+        for (int k = 0; k < b; ++k) a += (double)M[i * b + k] * x[k];
+        Zj[r * b + i] = a;
     }
 }
-// w -= sum_k h[k] V_k
-template <typename VT>
-__global__ void k_multi_axpy(int64_t n, int m, const double* __restrict__ h, const VT* __restrict__ V, VT* __restrict__ w) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double a = (double)w[i];
-    for (int k = 0; k < m; ++k) a -= h[k] * (double)V[(int64_t)k * n + i];
-    w[i] = (VT)a;
+
+// y = H^-1 gam over the cycle's G_J columns: column by column, one lane per two rows (one warp)
+__global__ void k_gm_y(double* G, int m) {
+    __shared__ double H[kGmMaxM * kGmMaxM];
+    const int jn = (int)G[G_J], lane = threadIdx.x;
+    for (int e = lane; e < jn * m; e += 32) H[e] = G[G_HES + e];
+    __syncwarp();
+    double r[2];   // the remaining right-hand side of rows lane and lane + 32
+#pragma unroll
+    for (int i = 0; i < 2; ++i) r[i] = lane + 32 * i < jn ? G[G_GAM + lane + 32 * i] : 0.0;
+    for (int k = jn - 1; k >= 0; --k) {
+        const double hkk = H[k * m + k];
+        const double yk = hkk != 0.0 ? __shfl_sync(0xffffffffu, k < 32 ? r[0] : r[1], k & 31) / hkk : 0.0;
+        if (lane == 0) G[G_Y + k] = yk;
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+            if (lane + 32 * i < k) r[i] -= H[(lane + 32 * i) * m + k] * yk;
+    }
 }
-// v = w / beta
-template <typename VT>
-__global__ void k_scale(int64_t n, const VT* __restrict__ w, double inv, VT* __restrict__ v) {
+
+// x += sum_k y[k] Z_k over the cycle's G_J columns   (Z = preconditioned basis)
+__global__ void k_gm_update(int64_t n, const double* __restrict__ G, const double* __restrict__ Z, double* __restrict__ x) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) v[i] = (VT)((double)w[i] * inv);
-}
-// x += sum_k y[k] Z_k   (Z = preconditioned basis)
-template <typename VT>
-__global__ void k_multi_axpy_add(int64_t n, int m, const double* __restrict__ y, const VT* __restrict__ Z, VT* __restrict__ x) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int jn = (int)G[G_J];
+    __shared__ double sh[kGmMaxM];
+    if (threadIdx.x < jn) sh[threadIdx.x] = G[G_Y + threadIdx.x];
+    __syncthreads();
     if (i >= n) return;
-    double a = (double)x[i];
-    for (int k = 0; k < m; ++k) a += y[k] * (double)Z[(int64_t)k * n + i];
-    x[i] = (VT)a;
+    double a = x[i];
+#pragma unroll 8
+    for (int k = 0; k < jn; ++k) a += sh[k] * Z[(int64_t)k * n + i];
+    x[i] = a;
 }
 
 static inline int grid_for(int64_t n, int t = 256) { return (int)((n + t - 1) / t); }
@@ -701,12 +1023,6 @@ static cudaError_t spmv(const Disc& D, const MT* vals, const VT* x, VT* y, cudaS
         k_bsr_mv<MT, VT, 3, G><<<grid_for(nR * G), 256, 0, s>>>(nR, D.d_rowPtr, D.d_colIdx, vals, x, y, gate);
     }
     return cudaGetLastError();
-}
-
-template <typename MT, typename VT>
-static void prec_apply(const Disc& D, const MT* Dinv, const VT* in, VT* out, cudaStream_t s) {
-    if (D.dim == 3) k_prec<MT, VT, 4><<<grid_for(D.nNodes), 256, 0, s>>>(D.nNodes, Dinv, in, out);
-    else k_prec<MT, VT, 3><<<grid_for(D.nNodes), 256, 0, s>>>(D.nNodes, Dinv, in, out);
 }
 
 template <typename VT, int K>
@@ -749,7 +1065,7 @@ bool Disc::ensure_workspace(int prec, int gmresM) {
     if (!al(ws.D, n * 8) || !al(ws.Dt, n * 8) || !al(ws.Ut, n * 8) || !al(ws.du, n * 8) ||
         !al(ws.J, colIdx.size() * b * b * vt) || !al(ws.Dinv, (size_t)nNodes * b * b * vt) ||
         !al(ws.vec, (size_t)nvec * n * sizeof(double)) || !al(ws.red, sizeof(double) * kRedBlocks * 80) ||
-        !al(ws.scal, sizeof(double) * 256))
+        !al(ws.scal, sizeof(double) * (kGmresScal + G_NSCAL)))
         return false;
     if (!cuda_ok(cudaMallocHost((void**)&ws.hscal, sizeof(double) * 256), "pinned alloc")) return false;
     ws.prec = prec; ws.n = n; ws.nvec = nvec; ws.gmresM = gmresM;
@@ -884,95 +1200,68 @@ static int bicgstab(Disc& D, const MT* J, const MT* Dinv, const double* rhs, dou
     return maxit;
 }
 
+// Iterations queued between two host reads of the solver state (as kBicgBatch): the kernels of
+// a later queued iteration return at once after a stop.
+static constexpr int kGmresBatch = 16;
+
 // restarted GMRES(m), right preconditioned, classical Gram-Schmidt with one
-// re-orthogonalisation pass; Hessenberg least squares (Givens) on the host.
+// re-orthogonalisation pass; Hessenberg least squares (Givens) on the device.
 template <typename MT>
 static int gmres(Disc& D, const MT* J, const MT* Dinv, const double* rhs, double* x, double rtol, int maxit, int m, double* relres, cudaStream_t s) {
-    using VT = double;
     Workspace& W = D.ws;
     const int64_t n = W.n;
-    VT* base = (VT*)W.vec;
-    VT* w = base;                 // work vector
-    VT* Vb = base + 1 * n;        // basis V_0..V_m
-    VT* Zb = base + (1 + m + 1) * n;   // preconditioned basis Z_0..Z_{m-1}
-    double* hdev = W.scal + 32;   // up to 64 + 1 coefficients
-    const int g = grid_for(n);
-    k_fill<VT><<<g, 256, 0, s>>>(n, x, VT(0));
-    std::vector<double> H((m + 1) * m), cs(m), sn(m), gam(m + 1), y(m);
-    double beta0 = -1.0;
-    int it = 0;
+    double* base = (double*)W.vec;
+    double* w = base;                      // J x at a restart
+    double* Vb = base + 1 * n;             // basis V_0..V_m
+    double* Zb = base + (1 + m + 1) * n;   // preconditioned basis Z_0..Z_{m-1}
+    double* G = W.scal + kGmresScal;
+    unsigned* counters = reinterpret_cast<unsigned*>(W.scal + 200);
+    const int g = grid_for(n), gRows = grid_for(D.nNodes, kGmT);
+    const int gRed = (int)std::min<int64_t>(kGmBlocks, (n + kGmT - 1) / kGmT);
+    const size_t smemMax = (size_t)(m + 1) * kGmT * sizeof(double);
+    if (!D.cuda_ok(cudaFuncSetAttribute(k_gm_axpy_dots, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemMax), "gmres setup")) return -1;
+    k_fill<double><<<g, 256, 0, s>>>(n, x, 0.0);
+    cudaMemsetAsync(G, 0, sizeof(double) * G_H1, s);
+    cudaMemsetAsync(counters, 0, 4 * sizeof(unsigned), s);
     *relres = 1.0;
+    int it = 0;
+    bool first = true;
     while (it < maxit) {
-        // V_0 = rhs - J x
-        spmv<MT, VT>(D, J, x, w, s);
-        cudaMemcpyAsync(Vb, rhs, n * sizeof(VT), cudaMemcpyDeviceToDevice, s);
-        W.hscal[40] = 1.0;
-        cudaMemcpyAsync(hdev, W.hscal + 40, sizeof(double), cudaMemcpyHostToDevice, s);
-        k_multi_axpy<VT><<<g, 256, 0, s>>>(n, 1, hdev, w, Vb);
-        {
-            const VT* a[1] = {Vb};
-            dots<VT, 1>(n, a, a, W.red, s);
-            k_dot_final<1><<<1, kRedThreads, 0, s>>>(W.red, kRedBlocks, W.scal + S_NR2);
+        // V_0 = rhs - J x (x = 0 in the first cycle)
+        if (!first) spmv<MT, double>(D, J, x, w, s);
+        k_gm_start<<<gRed, kGmT, 0, s>>>(n, rhs, first ? nullptr : w, Vb, W.red, counters, G, rtol);
+        first = false;
+        int j = 0, done = 0;
+        while (!done && j < m && it < maxit) {
+            const int K = std::min(std::min(kGmresBatch, m - j), maxit - it);
+            for (int q = 0; q < K; ++q, ++j) {
+                double* Vj = Vb + (int64_t)j * n;
+                double* Zj = Zb + (int64_t)j * n;
+                double* wj = Vj + n;
+                // the first of a batch finds iteration j - 1 ended already
+                const int jEnd = q > 0 ? j : 0;
+                if (D.dim == 3) k_gm_prec<MT, 4><<<gRows + 1, kGmT, 0, s>>>(D.nNodes, G, Vj, Dinv, Zj, jEnd, m, rtol);
+                else k_gm_prec<MT, 3><<<gRows + 1, kGmT, 0, s>>>(D.nNodes, G, Vj, Dinv, Zj, jEnd, m, rtol);
+                spmv<MT, double>(D, J, Zj, wj, s, G + G_DONE);
+                k_gm_dots<<<gRed, kGmT, 0, s>>>(n, j, Vb, wj, W.red, counters, G);
+                k_gm_axpy_dots<<<gRed, kGmT, (size_t)(j + 2) * kGmT * sizeof(double), s>>>(n, j, Vb, wj, W.red, counters, G);
+                k_gm_end<<<gRed, kGmT, 0, s>>>(n, j, Vb, wj, W.red, counters, G);
+            }
+            k_gm_givens<<<1, kGmT, 0, s>>>(G, j - 1, m, rtol);
+            if (!D.cuda_ok(cudaGetLastError(), "gmres launch")) return -1;
+            if (!D.cuda_ok(cudaMemcpyAsync(W.hscal, G, sizeof(double) * G_H1, cudaMemcpyDeviceToHost, s), "gmres state") ||
+                !D.cuda_ok(cudaStreamSynchronize(s), "gmres state"))
+                return -1;
+            done = (int)W.hscal[G_DONE];
+            it = (int)W.hscal[G_IT];
+            *relres = W.hscal[G_RELRES];
         }
-        if (!read_scal(D, S_NR2, 1, s)) return -1;
-        const double beta = std::sqrt(W.hscal[S_NR2]);
-        if (beta0 < 0) beta0 = beta;
-        if (beta0 == 0.0) return 0;
-        *relres = beta / beta0;
-        if (*relres < rtol) return it;
-        k_scale<VT><<<g, 256, 0, s>>>(n, Vb, 1.0 / beta, Vb);
-        std::fill(gam.begin(), gam.end(), 0.0);
-        gam[0] = beta;
-        int j = 0;
-        for (; j < m && it < maxit; ++j) {
-            ++it;
-            VT* Zj = Zb + (int64_t)j * n;
-            prec_apply<MT, VT>(D, Dinv, Vb + (int64_t)j * n, Zj, s);
-            spmv<MT, VT>(D, J, Zj, w, s);
-            double hcol[66] = {0};
-            for (int pass = 0; pass < 2; ++pass) {
-                k_multidot_partial<VT><<<kRedBlocks, kRedThreads, 0, s>>>(n, j + 1, Vb, w, W.red);
-                k_multidot_final<<<1, kRedThreads, 0, s>>>(W.red, kRedBlocks, j + 1, hdev);
-                k_multi_axpy<VT><<<g, 256, 0, s>>>(n, j + 1, hdev, Vb, w);
-                if (!D.cuda_ok(cudaMemcpyAsync(W.hscal + 64, hdev, sizeof(double) * (j + 1), cudaMemcpyDeviceToHost, s), "h")) return -1;
-                if (!D.cuda_ok(cudaStreamSynchronize(s), "sync")) return -1;
-                for (int k = 0; k <= j; ++k) hcol[k] += W.hscal[64 + k];
-            }
-            {
-                const VT* a[1] = {w};
-                dots<VT, 1>(n, a, a, W.red, s);
-                k_dot_final<1><<<1, kRedThreads, 0, s>>>(W.red, kRedBlocks, W.scal + S_NR2);
-            }
-            if (!read_scal(D, S_NR2, 1, s)) return -1;
-            const double hn = std::sqrt(W.hscal[S_NR2]);
-            hcol[j + 1] = hn;
-            if (hn > 0.0) k_scale<VT><<<g, 256, 0, s>>>(n, w, 1.0 / hn, Vb + (int64_t)(j + 1) * n);
-            // apply previous Givens rotations, then a new one
-            for (int k = 0; k < j; ++k) {
-                const double a = hcol[k], b2 = hcol[k + 1];
-                hcol[k] = cs[k] * a + sn[k] * b2;
-                hcol[k + 1] = -sn[k] * a + cs[k] * b2;
-            }
-            const double a = hcol[j], b2 = hcol[j + 1];
-            const double rr = std::sqrt(a * a + b2 * b2);
-            cs[j] = rr > 0 ? a / rr : 1.0; sn[j] = rr > 0 ? b2 / rr : 0.0;
-            hcol[j] = rr; hcol[j + 1] = 0.0;
-            gam[j + 1] = -sn[j] * gam[j];
-            gam[j] = cs[j] * gam[j];
-            for (int k = 0; k <= j; ++k) H[k * m + j] = hcol[k];
-            *relres = std::fabs(gam[j + 1]) / beta0;
-            if (!std::isfinite(*relres)) return -1;
-            if (*relres < rtol || hn == 0.0) { ++j; break; }
-        }
+        if (done == GM_NONFINITE) return -1;
+        const int jn = (int)W.hscal[G_J];
+        if (jn == 0) return it;   // zero right-hand side, or converged at the start of the cycle
         // y = H^-1 gam ; x += Z y
-        for (int k = j - 1; k >= 0; --k) {
-            double acc = gam[k];
-            for (int q = k + 1; q < j; ++q) acc -= H[k * m + q] * y[q];
-            y[k] = (H[k * m + k] != 0.0) ? acc / H[k * m + k] : 0.0;
-        }
-        std::memcpy(W.hscal + 64, y.data(), sizeof(double) * j);
-        cudaMemcpyAsync(hdev, W.hscal + 64, sizeof(double) * j, cudaMemcpyHostToDevice, s);
-        k_multi_axpy_add<VT><<<g, 256, 0, s>>>(n, j, hdev, Zb, x);
+        k_gm_y<<<1, 32, 0, s>>>(G, m);
+        k_gm_update<<<g, 256, 0, s>>>(n, G, Zb, x);
         if (!D.cuda_ok(cudaGetLastError(), "gmres launch")) return -1;
         if (*relres < rtol) return it;
     }

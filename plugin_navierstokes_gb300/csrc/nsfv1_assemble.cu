@@ -5,6 +5,7 @@
 // per entry is fixed (colour order, then SCVF order): runs are bitwise
 // reproducible.
 #include "nsfv1_asm_common.cuh"
+#include "nsfv1_tensor.cuh"
 
 namespace nsfv1 {
 
@@ -309,14 +310,55 @@ static cudaError_t dispatch_roid(int roid, F&& f) {
 // 152 SMs (the block size is a per-handle parameter picked by the autotuner).
 static int clamp_threads(int t) { return (t >= 32 && t <= kThreads && t % 32 == 0) ? t : kThreads; }
 
+// The tensor kernels on one colour: the affine elements, then the others. Returns the elements
+// they do not serve (LPS off the affine path) in 'rest' (count 0 if none).
+template <bool JAC>
+static cudaError_t launch_tensor(int roid, const DiscParams& P, const AsmArgs& a, cudaStream_t s, int threads, AsmArgs& rest) {
+    rest = a;
+    if ((roid != ROID_QUADRILATERAL && roid != ROID_HEXAHEDRON) || !tensor_params(P, JAC)) return cudaSuccess;
+    const int t = clamp_threads(threads);
+    auto part = [&](auto dim, auto flow, auto affine, const AsmArgs& q) {
+        constexpr int DIM = decltype(dim)::value;
+        using TN = Ten<DIM>;
+        if (q.count <= 0) return;
+        const int per = t / 32 * TN::EPW, grid = (q.count + per - 1) / per;
+        k_tensor<DIM, JAC, decltype(flow)::value, decltype(affine)::value>
+            <<<grid, t, (size_t)TN::warp_doubles(JAC) * (t / 32) * sizeof(double), s>>>(P, q);
+    };
+    auto both = [&](auto affine, const AsmArgs& q) {
+        const bool flow = P.stab == STAB_FLOW;
+        if (roid == ROID_HEXAHEDRON) {
+            if (flow) part(std::integral_constant<int, 3>{}, std::true_type{}, affine, q);
+            else part(std::integral_constant<int, 3>{}, std::false_type{}, affine, q);
+        } else {
+            if (flow) part(std::integral_constant<int, 2>{}, std::true_type{}, affine, q);
+            else part(std::integral_constant<int, 2>{}, std::false_type{}, affine, q);
+        }
+    };
+    AsmArgs q = a;
+    q.count = a.nAffine;
+    both(std::true_type{}, q);
+    q.elems = a.elems + a.nAffine;
+    q.count = a.count - a.nAffine;
+    rest = q;
+    if (P.convUpwind != UPW_LPS) {
+        both(std::false_type{}, q);
+        rest.count = 0;
+    }
+    return cudaGetLastError();
+}
+
 cudaError_t launch_defect(int roid, const DiscParams& P, const AsmArgs& a, cudaStream_t s, int threads) {
     if (a.count <= 0) return cudaSuccess;
     if (uses_ipshape(P)) return launch_defect_ipshape(roid, P, a, s);
+    AsmArgs q;
+    const cudaError_t e = launch_tensor<false>(roid, P, a, s, threads, q);
+    if (e != cudaSuccess || q.count <= 0) return e;
     const int t = clamp_threads(threads);
-    const int grid = (a.count + t - 1) / t;
+    const int grid = (q.count + t - 1) / t;
     return dispatch_roid(roid, [&](auto r) {
-        if (P.transient) k_defect<decltype(r)::value, true><<<grid, t, 0, s>>>(P, a);
-        else k_defect<decltype(r)::value, false><<<grid, t, 0, s>>>(P, a);
+        if (P.transient) k_defect<decltype(r)::value, true><<<grid, t, 0, s>>>(P, q);
+        else k_defect<decltype(r)::value, false><<<grid, t, 0, s>>>(P, q);
     });
 }
 
@@ -324,12 +366,15 @@ cudaError_t launch_jacobian(int roid, const DiscParams& P, const AsmArgs& a, int
     if (a.count <= 0) return cudaSuccess;
     if (uses_ipshape(P)) return launch_jacobian_ipshape(roid, P, a, prec, s);
     if (prec != 0) return launch_jacobian_lanes(roid, P, a, s);
+    AsmArgs q;
+    const cudaError_t e = launch_tensor<true>(roid, P, a, s, threads, q);
+    if (e != cudaSuccess || q.count <= 0) return e;
     const int t = clamp_threads(threads);
-    const int grid = (a.count + t - 1) / t;
+    const int grid = (q.count + t - 1) / t;
     return dispatch_roid(roid, [&](auto r) {
         constexpr int RO = decltype(r)::value;
-        if (P.pac && !P.stokes) k_jacobian<RO, double, double, true><<<grid, t, 0, s>>>(P, a);
-        else k_jacobian<RO, double, double, false><<<grid, t, 0, s>>>(P, a);
+        if (P.pac && !P.stokes) k_jacobian<RO, double, double, true><<<grid, t, 0, s>>>(P, q);
+        else k_jacobian<RO, double, double, false><<<grid, t, 0, s>>>(P, q);
     });
 }
 
@@ -346,17 +391,20 @@ cudaError_t launch_defect_jacobian(int roid, const DiscParams& P, const AsmArgs&
         const cudaError_t e = launch_defect(roid, P, a, s, threads);
         return e != cudaSuccess ? e : launch_jacobian_lanes(roid, P, a, s);
     }
+    AsmArgs q;
+    const cudaError_t e = launch_tensor<true>(roid, P, a, s, threads, q);
+    if (e != cudaSuccess || q.count <= 0) return e;
     const int t = clamp_threads(threads);
-    const int grid = (a.count + t - 1) / t;
+    const int grid = (q.count + t - 1) / t;
     return dispatch_roid(roid, [&](auto r) {
         constexpr int RO = decltype(r)::value;
         const bool pac = P.pac && !P.stokes;
         if (P.transient) {
-            if (pac) k_defect_jacobian<RO, true, true><<<grid, t, 0, s>>>(P, a);
-            else k_defect_jacobian<RO, true, false><<<grid, t, 0, s>>>(P, a);
+            if (pac) k_defect_jacobian<RO, true, true><<<grid, t, 0, s>>>(P, q);
+            else k_defect_jacobian<RO, true, false><<<grid, t, 0, s>>>(P, q);
         } else {
-            if (pac) k_defect_jacobian<RO, false, true><<<grid, t, 0, s>>>(P, a);
-            else k_defect_jacobian<RO, false, false><<<grid, t, 0, s>>>(P, a);
+            if (pac) k_defect_jacobian<RO, false, true><<<grid, t, 0, s>>>(P, q);
+            else k_defect_jacobian<RO, false, false><<<grid, t, 0, s>>>(P, q);
         }
     });
 }

@@ -275,6 +275,37 @@ static int build_coloring(int nsh, int64_t nNodes, int64_t nElems, const int32_t
     return nc;
 }
 
+// The affine test of elem_is_affine (nsfv1_elem.cuh) per element: simplices always, prisms
+// never, a quadrilateral / hexahedron when every corner is x0 plus edge vectors to within
+// 1e-14 of the element size (false when anything is NaN).
+static std::vector<uint8_t> affine_elements(int roid, int64_t nElems, const double* coords, const int32_t* conn) {
+    if (roid != ROID_QUADRILATERAL && roid != ROID_HEXAHEDRON) return std::vector<uint8_t>(nElems, roid == ROID_PRISM ? 0 : 1);
+    std::vector<uint8_t> aff(nElems);
+    const int dim = ref_dim(roid), nsh = ref_nsh(roid);
+    for (int64_t e = 0; e < nElems; ++e) {
+        const int32_t* c = conn + e * nsh;
+        auto x = [&](int k, int d) { return coords[(int64_t)c[k] * dim + d]; };
+        double sz = 0.0, dev = 0.0;
+        auto up = [](double& m, double v) { v = std::fabs(v); if (!(v <= m)) m = v; };   // keeps a NaN
+        for (int d = 0; d < dim; ++d) {
+            if (dim == 2) {
+                up(sz, x(1, d) - x(0, d));
+                up(sz, x(3, d) - x(0, d));
+                up(dev, (x(2, d) - x(1, d)) - (x(3, d) - x(0, d)));
+            } else {
+                const double a = x(1, d) - x(0, d), b = x(3, d) - x(0, d), g = x(4, d) - x(0, d);
+                up(sz, a); up(sz, b); up(sz, g);
+                up(dev, (x(2, d) - x(0, d)) - (a + b));
+                up(dev, (x(5, d) - x(0, d)) - (a + g));
+                up(dev, (x(7, d) - x(0, d)) - (b + g));
+                up(dev, (x(6, d) - x(0, d)) - (a + b + g));
+            }
+        }
+        aff[e] = dev <= 1e-14 * sz;
+    }
+    return aff;
+}
+
 }  // namespace nsfv1
 
 // ============================================================================
@@ -404,8 +435,13 @@ int nsfv1_set_mesh(nsfv1_disc* h, int elem_type, int64_t n_nodes, const double* 
         for (int c = 0; c < D->nColors; ++c) D->colorPtr[c + 1] += D->colorPtr[c];
         D->colorElems.resize(n_elems);
         {
+            // within a colour the affine elements first (their own kernels, nsfv1_tensor.cuh)
+            const std::vector<uint8_t> aff = affine_elements(elem_type, n_elems, coords, conn);
             std::vector<int32_t> f(D->colorPtr.begin(), D->colorPtr.end() - 1);
-            for (int64_t e = 0; e < n_elems; ++e) D->colorElems[f[D->color[e]]++] = (int32_t)e;
+            for (int64_t e = 0; e < n_elems; ++e) if (aff[e]) D->colorElems[f[D->color[e]]++] = (int32_t)e;
+            D->colorAffine.resize(D->nColors);
+            for (int c = 0; c < D->nColors; ++c) D->colorAffine[c] = f[c] - D->colorPtr[c];
+            for (int64_t e = 0; e < n_elems; ++e) if (!aff[e]) D->colorElems[f[D->color[e]]++] = (int32_t)e;
         }
         if (!D->cuda_ok(dupload(D->d_coords, coords, (size_t)n_nodes * dim), "upload coords") ||
             !D->cuda_ok(dupload(D->d_conn, conn, (size_t)n_elems * nsh), "upload conn") ||
@@ -996,7 +1032,7 @@ bool Disc::assemble_defect(const double* u, const double* u_old, double dt, doub
     if (!cuda_ok(cudaMemsetAsync(d, 0, sizeof(double) * nNodes * b, s), "memset defect")) return false;
     for (int c = 0; c < nColors; ++c) {
         AsmArgs a{d_coords, d_conn, d_elemBlk, d_colorElems + colorPtr[c], colorPtr[c + 1] - colorPtr[c], d_err, u, u_old, d, nullptr,
-                  d_nuElem, instSkip ? d_elemInst : nullptr, d_instActive, nNodes, (int64_t)colIdx.size()};
+                  d_nuElem, instSkip ? d_elemInst : nullptr, d_instActive, nNodes, (int64_t)colIdx.size(), colorAffine[c]};
         if (!cuda_ok(launch_defect(roid, P, a, s, asmThreads), "defect kernel")) return false;
     }
     if (!outflow_terms(P, u, d, nullptr, 0, s)) return false;
@@ -1019,7 +1055,7 @@ bool Disc::assemble_defect_jacobian(const double* u, const double* u_old, double
     if (!cuda_ok(cudaMemsetAsync(vals, 0, colIdx.size() * b * b * vsize, s), "memset jacobian")) return false;
     for (int c = 0; c < nColors; ++c) {
         AsmArgs a{d_coords, d_conn, d_elemBlk, d_colorElems + colorPtr[c], colorPtr[c + 1] - colorPtr[c], d_err, u, u_old, d, vals,
-                  d_nuElem, instSkip ? d_elemInst : nullptr, d_instActive, nNodes, (int64_t)colIdx.size()};
+                  d_nuElem, instSkip ? d_elemInst : nullptr, d_instActive, nNodes, (int64_t)colIdx.size(), colorAffine[c]};
         if (!cuda_ok(launch_defect_jacobian(roid, P, a, prec, s, asmThreads), "defect+jacobian kernel")) return false;
     }
     if (!outflow_terms(P, u, d, vals, prec, s)) return false;
@@ -1041,7 +1077,7 @@ bool Disc::assemble_jacobian(const double* u, const double* u_old, double dt, vo
     if (!cuda_ok(cudaMemsetAsync(vals, 0, bytes, s), "memset jacobian")) return false;
     for (int c = 0; c < nColors; ++c) {
         AsmArgs a{d_coords, d_conn, d_elemBlk, d_colorElems + colorPtr[c], colorPtr[c + 1] - colorPtr[c], d_err, u, u_old, nullptr, vals,
-                  d_nuElem, instSkip ? d_elemInst : nullptr, d_instActive, nNodes, (int64_t)colIdx.size()};
+                  d_nuElem, instSkip ? d_elemInst : nullptr, d_instActive, nNodes, (int64_t)colIdx.size(), colorAffine[c]};
         if (!cuda_ok(launch_jacobian(roid, P, a, prec, s, asmThreads), "jacobian kernel")) return false;
     }
     if (!outflow_terms(P, u, nullptr, vals, prec, s)) return false;

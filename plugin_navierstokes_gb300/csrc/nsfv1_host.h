@@ -41,6 +41,7 @@ struct Disc {
     int roid = 0, nsh = 0, nColors = 0;
     int64_t nNodes = 0, nElems = 0;
     std::vector<int32_t> rowPtr, colIdx, elemBlk, color, colorPtr, colorElems;
+    std::vector<int32_t> colorAffine;   // affine elements of each colour: they come first in its part of colorElems
     double* d_coords = nullptr;
     int32_t *d_conn = nullptr, *d_elemBlk = nullptr, *d_colorElems = nullptr, *d_rowPtr = nullptr, *d_colIdx = nullptr;
     int32_t* d_diagPos = nullptr;   // block index of each row's diagonal block

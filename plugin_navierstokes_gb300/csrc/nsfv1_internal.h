@@ -25,6 +25,7 @@ struct AsmArgs {
     const int32_t* instActive;// per-instance flag: elements of inactive instances are skipped
     int64_t nNodes = 0;       // index bounds checked by a build with NSFV1_BOUNDS_CHECK
     int64_t nnzb = 0;
+    int32_t nAffine = 0;      // elems[0, nAffine) have an affine reference mapping (elem_is_affine)
 };
 
 // Batched element-local callbacks (no global scatter).

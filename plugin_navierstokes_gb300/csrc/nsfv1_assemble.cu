@@ -6,6 +6,7 @@
 // reproducible.
 #include "nsfv1_asm_common.cuh"
 #include "nsfv1_tensor.cuh"
+#include "nsfv1_simplex.cuh"
 
 namespace nsfv1 {
 
@@ -310,13 +311,31 @@ static cudaError_t dispatch_roid(int roid, F&& f) {
 // 152 SMs (the block size is a per-handle parameter picked by the autotuner).
 static int clamp_threads(int t) { return (t >= 32 && t <= kThreads && t % 32 == 0) ? t : kThreads; }
 
-// The tensor kernels on one colour: the affine elements, then the others. Returns the elements
-// they do not serve (LPS off the affine path) in 'rest' (count 0 if none).
+// The specialised kernels on one colour: simplices, or the affine quadrilaterals / hexahedra and
+// then the others. Returns the elements they do not serve (prisms, LPS off the affine path, the
+// flags outside plain_params) in 'rest' (count 0 if none).
 template <bool JAC>
-static cudaError_t launch_tensor(int roid, const DiscParams& P, const AsmArgs& a, cudaStream_t s, int threads, AsmArgs& rest) {
+static cudaError_t launch_fast(int roid, const DiscParams& P, const AsmArgs& a, cudaStream_t s, int threads, AsmArgs& rest) {
     rest = a;
-    if ((roid != ROID_QUADRILATERAL && roid != ROID_HEXAHEDRON) || !tensor_params(P, JAC)) return cudaSuccess;
+    if (roid == ROID_PRISM || !plain_params(P, JAC)) return cudaSuccess;
     const int t = clamp_threads(threads);
+    if (roid == ROID_TRIANGLE || roid == ROID_TETRAHEDRON) {
+        const int grid = (a.count + t - 1) / t;
+        auto go = [&](auto dim, auto flow) {
+            constexpr int DIM = decltype(dim)::value;
+            k_simplex<DIM, JAC, decltype(flow)::value><<<grid, t, Simp<DIM>::smem_bytes(JAC, t), s>>>(P, a);
+        };
+        const bool flow = P.stab == STAB_FLOW;
+        if (roid == ROID_TRIANGLE) {
+            if (flow) go(std::integral_constant<int, 2>{}, std::true_type{});
+            else go(std::integral_constant<int, 2>{}, std::false_type{});
+        } else {
+            if (flow) go(std::integral_constant<int, 3>{}, std::true_type{});
+            else go(std::integral_constant<int, 3>{}, std::false_type{});
+        }
+        rest.count = 0;
+        return cudaGetLastError();
+    }
     auto part = [&](auto dim, auto flow, auto affine, const AsmArgs& q) {
         constexpr int DIM = decltype(dim)::value;
         using TN = Ten<DIM>;
@@ -352,7 +371,7 @@ cudaError_t launch_defect(int roid, const DiscParams& P, const AsmArgs& a, cudaS
     if (a.count <= 0) return cudaSuccess;
     if (uses_ipshape(P)) return launch_defect_ipshape(roid, P, a, s);
     AsmArgs q;
-    const cudaError_t e = launch_tensor<false>(roid, P, a, s, threads, q);
+    const cudaError_t e = launch_fast<false>(roid, P, a, s, threads, q);
     if (e != cudaSuccess || q.count <= 0) return e;
     const int t = clamp_threads(threads);
     const int grid = (q.count + t - 1) / t;
@@ -367,7 +386,7 @@ cudaError_t launch_jacobian(int roid, const DiscParams& P, const AsmArgs& a, int
     if (uses_ipshape(P)) return launch_jacobian_ipshape(roid, P, a, prec, s);
     if (prec != 0) return launch_jacobian_lanes(roid, P, a, s);
     AsmArgs q;
-    const cudaError_t e = launch_tensor<true>(roid, P, a, s, threads, q);
+    const cudaError_t e = launch_fast<true>(roid, P, a, s, threads, q);
     if (e != cudaSuccess || q.count <= 0) return e;
     const int t = clamp_threads(threads);
     const int grid = (q.count + t - 1) / t;
@@ -392,7 +411,7 @@ cudaError_t launch_defect_jacobian(int roid, const DiscParams& P, const AsmArgs&
         return e != cudaSuccess ? e : launch_jacobian_lanes(roid, P, a, s);
     }
     AsmArgs q;
-    const cudaError_t e = launch_tensor<true>(roid, P, a, s, threads, q);
+    const cudaError_t e = launch_fast<true>(roid, P, a, s, threads, q);
     if (e != cudaSuccess || q.count <= 0) return e;
     const int t = clamp_threads(threads);
     const int grid = (q.count + t - 1) / t;

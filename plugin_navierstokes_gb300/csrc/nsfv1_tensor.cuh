@@ -40,9 +40,9 @@
 
 namespace nsfv1 {
 
-// the calls the tensor kernels serve (everything else takes the kernels of nsfv1_elem.cuh);
+// the calls the tensor and simplex kernels serve (everything else takes the kernels of nsfv1_elem.cuh);
 // 'jac': the call forms the Jacobian
-inline bool tensor_params(const DiscParams& P, const bool jac) {
+inline bool plain_params(const DiscParams& P, const bool jac) {
     return !P.stokes && !P.laplace && !P.peclet && !P.pac && (!jac || P.fullNewton == 0.0) && P.diffLen == DL_RAW &&
            (P.stab == STAB_FIELDS || P.stab == STAB_FLOW) && P.sameUpwind &&
            (P.convUpwind == UPW_NO || P.convUpwind == UPW_FULL || P.convUpwind == UPW_LPS);

@@ -20,6 +20,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <vector>
 #include <cuda_bf16.h>
 #include <cudaTypedefs.h>
@@ -35,7 +36,8 @@ constexpr int kF = 16;        // Fourier frequencies
 constexpr int kIn0 = 4 * kF;  // 64 input features
 constexpr int kOut = 3;
 constexpr int kHeadPad = 64;  // head rows padded for the tensor-core tile
-constexpr int kRedChunks = 8; // point chunks per slot in the FiLM reductions
+constexpr int kOutPad = 4;    // FP32 head outputs of a point (three and a padding)
+constexpr int kBwdRows = 64;  // points of a block of the activation's backward pass
 
 __host__ __device__ constexpr int layer_in(int l) { return l == 0 ? kIn0 : kW; }
 
@@ -72,14 +74,28 @@ __device__ __forceinline__ uint64_t mix64(uint64_t z) {
     return z ^ (z >> 31);
 }
 
-__device__ __forceinline__ float sigmoid(float z) { return 1.0f / (1.0f + expf(-z)); }
+// 1 / x for x >= 1: the hardware estimate and one Newton-Raphson step in fused multiply-adds
+// (Markstein, "Computation of elementary functions on the IBM RISC System/6000", 1990).
+// Compared with the IEEE division for every float of [1, 1e37): the same bits; beyond, where
+// |z / x| < 1e-34, within one unit in the last place. Without the division's branch,
+// which kept neighbouring elements of the activation from overlapping.
+__device__ __forceinline__ float recip_ge1(float x) {
+    float r;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+    const float e = fmaf(-x, r, 1.0f), q = fmaf(r, e, r);
+    return x < 1.0e38f ? q : r;   // x = inf: r = 0
+}
+
+__device__ __forceinline__ float sigmoid(float z) { return recip_ge1(1.0f + expf(-z)); }
 
 // ---- kernels ----------------------------------------------------------------
 
-// features of points [0, P) (rows P..Pp-1 zero): h0 [Pp x 64] and h0T [64 x Pp]
-__global__ void k_features(int64_t P, int64_t Pp, const float2* __restrict__ xy, bf16* __restrict__ h0, bf16* __restrict__ h0T) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int k = blockIdx.y;   // frequency index 0..15
+// features of points [0, P) (rows P..Pp-1 zero): h0 [Pp x 64]. One thread per point and
+// frequency, the 16 frequencies of a point on consecutive lanes: 128-byte rows are written
+// whole (with one frequency per block and single 2-byte stores it took 89 us for 33 k points).
+__global__ void k_features(int64_t P, int64_t Pp, const float2* __restrict__ xy, bf16* __restrict__ h0) {
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, i = t / kF;
+    const int k = (int)(t % kF);
     if (i >= Pp) return;
     float v[4] = {0.f, 0.f, 0.f, 0.f};
     if (i < P) {
@@ -87,12 +103,8 @@ __global__ void k_features(int64_t P, int64_t Pp, const float2* __restrict__ xy,
         sincospif((float)(k + 1) * p.x, &v[0], &v[1]);
         sincospif((float)(k + 1) * p.y, &v[2], &v[3]);
     }
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        const bf16 h = __float2bfloat16(v[c]);
-        h0[i * kIn0 + 4 * k + c] = h;
-        h0T[(int64_t)(4 * k + c) * Pp + i] = h;
-    }
+    __nv_bfloat162 o[2] = {{__float2bfloat16(v[0]), __float2bfloat16(v[1])}, {__float2bfloat16(v[2]), __float2bfloat16(v[3])}};
+    reinterpret_cast<uint2*>(h0)[i * kF + k] = *reinterpret_cast<const uint2*>(o);
 }
 
 // per-slot FiLM: gb[s][l][0..255] = gamma, gb[s][l][256..511] = beta
@@ -106,113 +118,138 @@ __global__ void k_film(int nSlots, const float* __restrict__ cond, const float* 
     gb[((int64_t)s * kL + l) * 2 * kW + kW + j] = be;
 }
 
-// h_{l+1} = silu(gamma (a + b) + beta) for rows < P (0 beyond), row-major and transposed.
-// block (32, 8), tile 32 points x 32 features
-__global__ void k_act_fwd(int64_t P, int64_t Pp, int l, const float* __restrict__ a, const float* __restrict__ prm, Offsets off,
-                          const float* __restrict__ gb, const int32_t* __restrict__ pointSlot, bf16* __restrict__ h,
-                          bf16* __restrict__ hT) {
-    __shared__ bf16 tile[32][33];
-    const int64_t i0 = blockIdx.x * 32ll;
-    const int j = blockIdx.y * 32 + threadIdx.x;
-    const float bj = prm[off.b[l] + j];
-    for (int r = threadIdx.y; r < 32; r += 8) {
-        const int64_t i = i0 + r;
-        float hv = 0.f;
-        if (i < P) {
-            const float* g = gb + ((int64_t)pointSlot[i] * kL + l) * 2 * kW;
-            const float z = g[j] * (a[i * kW + j] + bj) + g[kW + j];
-            hv = z * sigmoid(z);
-        }
-        const bf16 hb = __float2bfloat16(hv);
-        h[i * kW + j] = hb;
-        tile[r][threadIdx.x] = hb;
+// the activation of k_layer: silu(gamma (a + b) + beta), packed to BF16 pairs
+struct SiluFilm {
+    __device__ __forceinline__ float operator()(float a, float b, float g, float be) const {
+        const float z = g * (a + b) + be;
+        return z * sigmoid(z);
     }
-    __syncthreads();
-    for (int r = threadIdx.y; r < 32; r += 8) hT[(int64_t)(blockIdx.y * 32 + r) * Pp + i0 + threadIdx.x] = tile[threadIdx.x][r];
-}
-
-// da = dh * silu'(z) * gamma (BF16, row-major and transposed; 0 for rows >= P)
-__global__ void k_act_bwd(int64_t P, int64_t Pp, int l, const float* __restrict__ a, const float* __restrict__ dh,
-                          const float* __restrict__ prm, Offsets off, const float* __restrict__ gb,
-                          const int32_t* __restrict__ pointSlot, bf16* __restrict__ da, bf16* __restrict__ daT) {
-    __shared__ bf16 tile[32][33];
-    const int64_t i0 = blockIdx.x * 32ll;
-    const int j = blockIdx.y * 32 + threadIdx.x;
-    const float bj = prm[off.b[l] + j];
-    for (int r = threadIdx.y; r < 32; r += 8) {
-        const int64_t i = i0 + r;
-        float v = 0.f;
-        if (i < P) {
-            const float* g = gb + ((int64_t)pointSlot[i] * kL + l) * 2 * kW;
-            const float z = g[j] * (a[i * kW + j] + bj) + g[kW + j];
-            const float sg = sigmoid(z);
-            v = dh[i * kW + j] * sg * (1.0f + z * (1.0f - sg)) * g[j];
-        }
-        const bf16 vb = __float2bfloat16(v);
-        da[i * kW + j] = vb;
-        tile[r][threadIdx.x] = vb;
+    __device__ __forceinline__ uint32_t pack(float lo, float hi) const {
+        const __nv_bfloat162 v = {__float2bfloat16(lo), __float2bfloat16(hi)};
+        return *reinterpret_cast<const uint32_t*>(&v);
     }
-    __syncthreads();
-    for (int r = threadIdx.y; r < 32; r += 8) daT[(int64_t)(blockIdx.y * 32 + r) * Pp + i0 + threadIdx.x] = tile[threadIdx.x][r];
-}
+};
 
-// per (slot, chunk) partial sums over the chunk's points of
-//   dgamma = dz (a + b), dbeta = dz, db = dz gamma   (dz = dh silu'(z))
-__global__ void k_slot_red(int l, const int32_t* __restrict__ slotPtr, const float* __restrict__ a, const float* __restrict__ dh,
-                           const float* __restrict__ prm, Offsets off, const float* __restrict__ gb, float* __restrict__ part) {
-    const int s = blockIdx.x, c = blockIdx.y, j = threadIdx.x;
-    const int64_t p0 = slotPtr[s], p1 = slotPtr[s + 1];
-    const int64_t len = p1 - p0;
-    const int64_t q0 = p0 + len * c / kRedChunks, q1 = p0 + len * (c + 1) / kRedChunks;
-    const float* g = gb + ((int64_t)s * kL + l) * 2 * kW;
-    const float gj = g[j], bej = g[kW + j], bj = prm[off.b[l] + j];
-    float sg_ = 0.f, sb_ = 0.f, sd_ = 0.f;
-    for (int64_t i = q0; i < q1; ++i) {
-        const float ab = a[i * kW + j] + bj;
-        const float z = gj * ab + bej;
+// Backward pass of an activation over 64 points per block, two columns per thread:
+//   dz = dh silu'(z),  da = dz gamma (BF16; 0 for rows >= P),
+// and the sums over the block's points of each slot of dz (a + b), dz and dz gamma, which go to
+// part[block + slot] (blocks and slots both increase along the points, so the index is unique).
+// One pass over a and dh for everything that the separate activation and reduction kernels
+// (and the transposed copy of da) read twice: it is bound by that traffic.
+__global__ void __launch_bounds__(kW / 2) k_act_bwd(int64_t P, int l, const float* __restrict__ a, const float* __restrict__ dh,
+                                                    const float* __restrict__ prm, Offsets off, const float* __restrict__ gb,
+                                                    const int32_t* __restrict__ pointSlot, bf16* __restrict__ da, float* __restrict__ part) {
+    constexpr int U = 8;
+    const int j = 2 * threadIdx.x;
+    const int64_t i0 = (int64_t)blockIdx.x * kBwdRows;
+    const float2 b = *reinterpret_cast<const float2*>(prm + off.b[l] + j);
+    float s[3][2] = {};
+    float2 g = {0.f, 0.f}, be = {0.f, 0.f};
+    int slot = -1;
+    auto flush = [&]() {
+        float* o = part + ((int64_t)blockIdx.x + slot) * 3 * kW;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) *reinterpret_cast<float2*>(o + q * kW + j) = make_float2(s[q][0], s[q][1]);
+    };
+    auto back = [&](float ai, float di, float bi, float gi, float bei, float (&acc)[3][2], int c) {
+        const float ab = ai + bi;
+        const float z = gi * ab + bei;
         const float sg = sigmoid(z);
-        const float dz = dh[i * kW + j] * sg * (1.0f + z * (1.0f - sg));
-        sg_ += dz * ab;
-        sb_ += dz;
-        sd_ += dz * gj;
-    }
-    float* o = part + ((int64_t)s * kRedChunks + c) * 3 * kW;
-    o[j] = sg_;
-    o[kW + j] = sb_;
-    o[2 * kW + j] = sd_;
-}
-
-// FiLM and bias gradients of layer l from the per-slot partials (fixed order)
-__global__ void k_film_grad(int l, int nSlots, const float* __restrict__ cond, const float* __restrict__ part, Offsets off,
-                            float* __restrict__ grad) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= kW) return;
-    float gw0 = 0.f, gw1 = 0.f, gbs = 0.f, bw0 = 0.f, bw1 = 0.f, bbs = 0.f, db = 0.f;
-    for (int s = 0; s < nSlots; ++s) {
-        float dg = 0.f, dbe = 0.f;
-        for (int c = 0; c < kRedChunks; ++c) {
-            const float* o = part + ((int64_t)s * kRedChunks + c) * 3 * kW;
-            dg += o[j];
-            dbe += o[kW + j];
-            db += o[2 * kW + j];
+        const float dz = di * sg * (1.0f + z * (1.0f - sg));
+        const float v = dz * gi;
+        acc[0][c] += dz * ab;
+        acc[1][c] += dz;
+        acc[2][c] += v;
+        return v;
+    };
+    for (int r0 = 0; r0 < kBwdRows; r0 += U) {
+        float2 av[U], dv[U];
+        int sl[U];
+#pragma unroll
+        for (int r = 0; r < U; ++r) {
+            const int64_t i = i0 + r0 + r;
+            av[r] = dv[r] = make_float2(0.f, 0.f);
+            sl[r] = -1;
+            if (i < P) {
+                av[r] = *reinterpret_cast<const float2*>(a + i * kW + j);
+                dv[r] = *reinterpret_cast<const float2*>(dh + i * kW + j);
+                sl[r] = pointSlot[i];
+            }
         }
-        const float c0 = cond[2 * s], c1 = cond[2 * s + 1];
-        gw0 += dg * c0; gw1 += dg * c1; gbs += dg;
-        bw0 += dbe * c0; bw1 += dbe * c1; bbs += dbe;
+#pragma unroll
+        for (int r = 0; r < U; ++r) {
+            float v0 = 0.f, v1 = 0.f;
+            if (sl[r] >= 0) {
+                if (sl[r] != slot) {
+                    if (slot >= 0) flush();
+                    slot = sl[r];
+                    const float* f = gb + ((int64_t)slot * kL + l) * 2 * kW;
+                    g = *reinterpret_cast<const float2*>(f + j);
+                    be = *reinterpret_cast<const float2*>(f + kW + j);
+#pragma unroll
+                    for (int q = 0; q < 3; ++q) s[q][0] = s[q][1] = 0.f;
+                }
+                v0 = back(av[r].x, dv[r].x, b.x, g.x, be.x, s, 0);
+                v1 = back(av[r].y, dv[r].y, b.y, g.y, be.y, s, 1);
+            }
+            const __nv_bfloat162 o = {__float2bfloat16(v0), __float2bfloat16(v1)};
+            *reinterpret_cast<__nv_bfloat162*>(da + (i0 + r0 + r) * kW + j) = o;
+        }
     }
-    grad[off.Gw[l] + 2 * j] = gw0;
-    grad[off.Gw[l] + 2 * j + 1] = gw1;
-    grad[off.Gb[l] + j] = gbs;
-    grad[off.Bw[l] + 2 * j] = bw0;
-    grad[off.Bw[l] + 2 * j + 1] = bw1;
-    grad[off.Bb[l] + j] = bbs;
-    grad[off.b[l] + j] = db;
+    if (slot >= 0) flush();
 }
 
-// head: residual r = out + bh - target (points < P), dout = 2 r / (3 P) as BF16 [Pp x 64] and [64 x Pp];
+// per slot and layer: the partial sums of its blocks in order -> slotSum[l][s] (dgamma, dbeta, db)
+__global__ void k_slot_sum(const int32_t* __restrict__ slotPtr, const float* __restrict__ part, int64_t layerStride, float* __restrict__ slotSum) {
+    const int s = blockIdx.x, l = blockIdx.y, j = threadIdx.x;
+    const int b0 = slotPtr[s] / kBwdRows, b1 = (slotPtr[s + 1] - 1) / kBwdRows;
+    float v[3] = {0.f, 0.f, 0.f};
+#pragma unroll 8
+    for (int b = b0; b <= b1; ++b) {
+        const float* o = part + l * layerStride + ((int64_t)b + s) * 3 * kW;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) v[q] += o[q * kW + j];
+    }
+    float* o = slotSum + ((int64_t)l * gridDim.x + s) * 3 * kW;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) o[q * kW + j] = v[q];
+}
+
+// FiLM and bias gradients from the per-slot sums (fixed order): block (32 columns, 8 slot groups)
+__global__ void k_film_grad(int nSlots, const float* __restrict__ cond, const float* __restrict__ slotSum, Offsets off,
+                            float* __restrict__ grad) {
+    __shared__ float sh[7][8][32];
+    const int l = blockIdx.y, c = threadIdx.x, j = blockIdx.x * 32 + c;
+    float v[7] = {};
+#pragma unroll 4
+    for (int s = threadIdx.y; s < nSlots; s += 8) {
+        const float* o = slotSum + ((int64_t)l * nSlots + s) * 3 * kW;
+        const float c0 = cond[2 * s], c1 = cond[2 * s + 1], dg = o[j], dbe = o[kW + j];
+        v[0] += dg * c0; v[1] += dg * c1; v[2] += dg;
+        v[3] += dbe * c0; v[4] += dbe * c1; v[5] += dbe;
+        v[6] += o[2 * kW + j];
+    }
+#pragma unroll
+    for (int q = 0; q < 7; ++q) sh[q][threadIdx.y][c] = v[q];
+    __syncthreads();
+    if (threadIdx.y != 0) return;
+#pragma unroll
+    for (int q = 0; q < 7; ++q)
+#pragma unroll
+        for (int y = 1; y < 8; ++y) v[q] += sh[q][y][c];
+    grad[off.Gw[l] + 2 * j] = v[0];
+    grad[off.Gw[l] + 2 * j + 1] = v[1];
+    grad[off.Gb[l] + j] = v[2];
+    grad[off.Bw[l] + 2 * j] = v[3];
+    grad[off.Bw[l] + 2 * j + 1] = v[4];
+    grad[off.Bb[l] + j] = v[5];
+    grad[off.b[l] + j] = v[6];
+}
+
+// head: residual r = out + bh - target (points < P), dout = 2 r / (3 P) as BF16 [Pp x 64] (columns 3.. stay zero);
 // per-block partial sums of r^2 and of dout (the bias gradient), fixed order
 __global__ void k_head_loss(int64_t P, int64_t Pp, const float* __restrict__ out, const float* __restrict__ prm, Offsets off,
-                            const float* __restrict__ target, bf16* __restrict__ dout, bf16* __restrict__ doutT,
+                            const float* __restrict__ target, bf16* __restrict__ dout,
                             double* __restrict__ lossPart, float* __restrict__ dbhPart) {
     __shared__ double sl[256];
     __shared__ float sb[3][256];
@@ -223,7 +260,7 @@ __global__ void k_head_loss(int64_t P, int64_t Pp, const float* __restrict__ out
         const float scale = 2.0f / (3.0f * (float)P);
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            const float r = out[i * kHeadPad + c] + prm[off.bh + c] - target[i * 3 + c];
+            const float r = out[i * kOutPad + c] + prm[off.bh + c] - target[i * 3 + c];
             l2 += (double)r * r;
             d[c] = scale * r;
         }
@@ -231,9 +268,7 @@ __global__ void k_head_loss(int64_t P, int64_t Pp, const float* __restrict__ out
     if (i < Pp) {
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            const bf16 v = __float2bfloat16(d[c]);
-            dout[i * kHeadPad + c] = v;
-            doutT[(int64_t)c * Pp + i] = v;
+            dout[i * kHeadPad + c] = __float2bfloat16(d[c]);
         }
     }
     sl[threadIdx.x] = l2;
@@ -252,18 +287,29 @@ __global__ void k_head_loss(int64_t P, int64_t Pp, const float* __restrict__ out
     }
 }
 
+// loss and head bias gradient from the block sums: one block of 256 threads, fixed order
 __global__ void k_head_reduce(int nBlocks, int64_t P, const double* __restrict__ lossPart, const float* __restrict__ dbhPart,
                               Offsets off, float* __restrict__ grad, double* __restrict__ loss) {
-    if (threadIdx.x == 0) {
-        double s = 0.0;
-        for (int b = 0; b < nBlocks; ++b) s += lossPart[b];
-        *loss = s / (3.0 * (double)P);
+    __shared__ double sl[256];
+    __shared__ float sb[3][256];
+    double s = 0.0;
+    float d[3] = {0.f, 0.f, 0.f};
+    for (int b = threadIdx.x; b < nBlocks; b += 256) {
+        s += lossPart[b];
+        for (int c = 0; c < 3; ++c) d[c] += dbhPart[b * 3 + c];
     }
-    if (threadIdx.x < 3) {
-        float s = 0.f;
-        for (int b = 0; b < nBlocks; ++b) s += dbhPart[b * 3 + threadIdx.x];
-        grad[off.bh + threadIdx.x] = s;
+    sl[threadIdx.x] = s;
+    for (int c = 0; c < 3; ++c) sb[c][threadIdx.x] = d[c];
+    __syncthreads();
+    for (int w = 128; w > 0; w >>= 1) {
+        if (threadIdx.x < w) {
+            sl[threadIdx.x] += sl[threadIdx.x + w];
+            for (int c = 0; c < 3; ++c) sb[c][threadIdx.x] += sb[c][threadIdx.x + w];
+        }
+        __syncthreads();
     }
+    if (threadIdx.x == 0) *loss = sl[0] / (3.0 * (double)P);
+    if (threadIdx.x < 3) grad[off.bh + threadIdx.x] = sb[threadIdx.x][0];
 }
 
 // sum of split-K partials part[z][M][N] into dst (row-major M x N), fixed order
@@ -355,8 +401,8 @@ __global__ void k_write_state(int64_t P, int64_t i0, const float* __restrict__ o
                               float* __restrict__ outF) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= P) return;
-    const float o0 = out[i * kHeadPad] + prm[off.bh], o1 = out[i * kHeadPad + 1] + prm[off.bh + 1],
-                o2 = out[i * kHeadPad + 2] + prm[off.bh + 2];
+    const float4 v = reinterpret_cast<const float4*>(out)[i];
+    const float o0 = v.x + prm[off.bh], o1 = v.y + prm[off.bh + 1], o2 = v.z + prm[off.bh + 2];
     if (outF) {
         outF[(i0 + i) * 3] = o0;
         outF[(i0 + i) * 3 + 1] = o1;
@@ -407,15 +453,15 @@ bool make_map(CUtensorMap* m, const void* ptr, int64_t rows, int64_t K, int boxR
               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int BN, int STAGES>
+template <int BN, int STAGES, bool MN = false, bool HEAD = false>
 cudaError_t launch_gemm(const CUtensorMap& a, const CUtensorMap& b, float* C, int M, int N, int K, int splits, int kChunk, int* err,
                         cudaStream_t s) {
     using S = nsfv1::tc::GemmSmem<BN, STAGES>;
     // per launch: the attribute belongs to the current device
-    cudaError_t e = cudaFuncSetAttribute(nsfv1::tc::k_gemm_bf16_tn<BN, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kBytes);
+    cudaError_t e = cudaFuncSetAttribute(nsfv1::tc::k_gemm_bf16_tn<BN, STAGES, MN, HEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kBytes);
     if (e != cudaSuccess) return e;
     dim3 grid(M / nsfv1::tc::BM, N / BN, splits);
-    nsfv1::tc::k_gemm_bf16_tn<BN, STAGES><<<grid, 128, S::kBytes, s>>>(a, b, C, M, N, K, kChunk, err);
+    nsfv1::tc::k_gemm_bf16_tn<BN, STAGES, MN, HEAD><<<grid, 128, S::kBytes, s>>>(a, b, C, M, N, K, kChunk, err);
     return cudaGetLastError();
 }
 
@@ -442,6 +488,47 @@ int gemm_bf16(const bf16* A, const bf16* B, float* C, int M, int N, int K, int s
     return splits;
 }
 
+// C[splits][M][N] = A[K x M]^T * B[K x N], both row-major (the weight gradients: K = points).
+// M a multiple of 128, N 64 or 256, K of 64; as gemm_bf16 otherwise.
+int gemm_bf16_mn(const bf16* A, const bf16* B, float* C, int M, int N, int K, int splits, int* err, cudaStream_t s, std::string& why) {
+    const int kTiles = K / 64;
+    splits = std::min(splits, kTiles);
+    const int chunkTiles = (kTiles + splits - 1) / splits;
+    splits = (kTiles + chunkTiles - 1) / chunkTiles;
+    CUtensorMap ma, mb;
+    if (!make_map(&ma, A, K, M, 64) || !make_map(&mb, B, K, N, 64)) { why = "gemm: tensor map encoding failed"; return -1; }
+    const cudaError_t e = N == 64 ? launch_gemm<64, 6, true>(ma, mb, C, M, N, K, splits, chunkTiles * 64, err, s)
+                                  : launch_gemm<256, 4, true>(ma, mb, C, M, N, K, splits, chunkTiles * 64, err, s);
+    if (e != cudaSuccess) { why = std::string("gemm launch: ") + cudaGetErrorString(e); return -1; }
+    return splits;
+}
+
+// one layer (k_layer): with ACT h_out [Pp x 256], and a [Pp x 256] if given
+template <int K, bool ACT, bool STORE_A>
+cudaError_t launch_layer_k(const CUtensorMap& mh, const CUtensorMap& mw, const nsfv1::tc::LayerArgs& a, int sms, cudaStream_t s) {
+    using S = nsfv1::tc::LayerSmem<K>;
+    auto kern = nsfv1::tc::k_layer<K, ACT, STORE_A, SiluFilm>;
+    // per launch: the attribute belongs to the current device
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kBytes);
+    if (e != cudaSuccess) return e;
+    kern<<<std::min(a.nTiles, sms), S::THREADS, S::kBytes, s>>>(mh, mw, a, SiluFilm{});
+    return cudaGetLastError();
+}
+
+// h [Pp x K], W [256 x K]; a.h null: the product alone
+bool launch_layer(const bf16* h, const bf16* W, int K, int64_t Pp, const nsfv1::tc::LayerArgs& a, int sms, cudaStream_t s, std::string& why) {
+    CUtensorMap mh, mw;
+    if (!make_map(&mh, h, Pp, K, nsfv1::tc::BM) || !make_map(&mw, W, kW, K, kW)) { why = "mlp layer: tensor map encoding failed"; return false; }
+    auto go = [&](auto k) {
+        constexpr int KK = decltype(k)::value;
+        if (!a.h) return launch_layer_k<KK, false, true>(mh, mw, a, sms, s);
+        return a.a ? launch_layer_k<KK, true, true>(mh, mw, a, sms, s) : launch_layer_k<KK, true, false>(mh, mw, a, sms, s);
+    };
+    const cudaError_t e = K == kIn0 ? go(std::integral_constant<int, kIn0>{}) : go(std::integral_constant<int, kW>{});
+    if (e != cudaSuccess) { why = std::string("mlp layer launch: ") + cudaGetErrorString(e); return false; }
+    return true;
+}
+
 int g_num_sms() {
     int dev = 0, n = 0;
     cudaGetDevice(&dev);
@@ -459,10 +546,10 @@ struct nsfv1_mlp {
     int maxSlots = 0;
     float *prm = nullptr, *grad = nullptr, *am = nullptr, *av = nullptr;
     bf16 *W[kL] = {}, *WT[kL] = {}, *Wh = nullptr, *WhT = nullptr;
-    bf16 *h[kL + 1] = {}, *hT[kL + 1] = {};
+    bf16* h[kL + 1] = {};
     float* a[kL] = {};
-    float *out = nullptr, *dh = nullptr, *gb = nullptr, *part = nullptr, *splitBuf = nullptr, *cond = nullptr, *lid = nullptr;
-    bf16 *dout = nullptr, *doutT = nullptr, *da = nullptr, *daT = nullptr;
+    float *out = nullptr, *dh = nullptr, *gb = nullptr, *part = nullptr, *slotSum = nullptr, *splitBuf = nullptr, *cond = nullptr, *lid = nullptr;
+    bf16 *dout = nullptr, *da = nullptr;
     float *dbhPart = nullptr, *tgt = nullptr;
     float2* xy = nullptr;
     double *lossPart = nullptr, *loss = nullptr;
@@ -470,14 +557,17 @@ struct nsfv1_mlp {
     int* err = nullptr;
     int64_t adamStep = 0;
     size_t splitCap = 0;
+    int sms = 152;
+    // floats of one layer's backward partials (block + slot indexed)
+    int64_t part_stride() const { return (cap / kBwdRows + maxSlots) * 3 * kW; }
     std::string lastError;
 
     ~nsfv1_mlp() {
         auto f = [](auto*& p) { if (p) cudaFree((void*)p); p = nullptr; };
         f(prm); f(grad); f(am); f(av); f(Wh); f(WhT);
         for (int l = 0; l < kL; ++l) { f(W[l]); f(WT[l]); f(a[l]); }
-        for (int l = 0; l <= kL; ++l) { f(h[l]); f(hT[l]); }
-        f(out); f(dh); f(gb); f(part); f(splitBuf); f(cond); f(lid); f(dout); f(doutT); f(da); f(daT); f(dbhPart); f(tgt); f(xy);
+        for (int l = 0; l <= kL; ++l) f(h[l]);
+        f(out); f(dh); f(gb); f(part); f(slotSum); f(splitBuf); f(cond); f(lid); f(dout); f(da); f(dbhPart); f(tgt); f(xy);
         f(lossPart); f(loss); f(slotPtr); f(pointSlot); f(err);
     }
     int fail(int code, const std::string& m) { lastError = m; return code; }
@@ -489,13 +579,21 @@ struct nsfv1_mlp {
         k_refresh<<<dim3((kW * kW + 255) / 256, kL + 1), 256, 0, s>>>(prm, off, W[0], W[1], W[2], W[3], WT[0], WT[1], WT[2], WT[3], Wh, WhT);
         return cuda(cudaGetLastError(), "mlp weights");
     }
-    int gemm(const bf16* A, const bf16* B, float* C, int M, int N, int K, int splits, cudaStream_t s, int* used = nullptr) {
+    // dh [Pp x 256] = x [Pp x K] W [256 x K]^T
+    int product(const bf16* x, const bf16* W, int K, int64_t Pp, cudaStream_t s) {
+        nsfv1::tc::LayerArgs a{};
+        a.P = Pp; a.nTiles = (int)(Pp / 128); a.a = dh; a.err = err;
         std::string why;
-        if (C == splitBuf && (size_t)nsfv1_gemm_bf16_splits(K, splits) * M * N * 4 > splitCap)
+        if (!launch_layer(x, W, K, Pp, a, sms, s, why)) return fail(NSFV1_ERR_ARGUMENT, why);
+        return NSFV1_OK;
+    }
+    int gemm_mn(const bf16* A, const bf16* B, int N, int K, int splits, cudaStream_t s, int* used) {
+        std::string why;
+        if ((size_t)nsfv1_gemm_bf16_splits(K, splits) * kW * N * 4 > splitCap)
             return fail(NSFV1_ERR_ARGUMENT, "mlp: split-K partials exceed the staging buffer");
-        const int u = gemm_bf16(A, B, C, M, N, K, splits, err, s, why);
+        const int u = gemm_bf16_mn(A, B, splitBuf, kW, N, K, splits, err, s, why);
         if (u < 0) return fail(NSFV1_ERR_ARGUMENT, why);
-        if (used) *used = u;
+        *used = u;
         return NSFV1_OK;
     }
     int check_err(cudaStream_t s) {
@@ -509,19 +607,26 @@ struct nsfv1_mlp {
         }
         return NSFV1_OK;
     }
-    // forward of P <= cap points whose xy / pointSlot / gb are in place
-    int forward(int64_t P, cudaStream_t s) {
+    // forward of P <= cap points whose xy / pointSlot / gb are in place; keepA: the FP32
+    // pre-activations too (the backward pass reads them)
+    int forward(int64_t P, cudaStream_t s, bool keepA) {
         const int64_t Pp = (P + 127) / 128 * 128;
-        k_features<<<dim3((unsigned)((Pp + 255) / 256), kF), 256, 0, s>>>(P, Pp, xy, h[0], hT[0]);
+        k_features<<<(unsigned)(Pp * kF / 256), 256, 0, s>>>(P, Pp, xy, h[0]);
+        std::string why;
         for (int l = 0; l < kL; ++l) {
-            if (int st = gemm(h[l], W[l], a[l], (int)Pp, kW, layer_in(l), 1, s)) return st;
-            k_act_fwd<<<dim3((unsigned)(Pp / 32), kW / 32), dim3(32, 8), 0, s>>>(P, Pp, l, a[l], prm, off, gb, pointSlot, h[l + 1], hT[l + 1]);
+            const nsfv1::tc::LayerArgs a{P, (int)(Pp / 128), prm + off.b[l], gb + (int64_t)l * 2 * kW, (int64_t)kL * 2 * kW, pointSlot,
+                                         reinterpret_cast<uint16_t*>(h[l + 1]), keepA ? this->a[l] : nullptr, err};
+            if (!launch_layer(h[l], W[l], layer_in(l), Pp, a, sms, s, why)) return fail(NSFV1_ERR_ARGUMENT, why);
         }
-        if (int st = gemm(h[kL], Wh, out, (int)Pp, kHeadPad, kW, 1, s)) return st;
+        // the head: four stages hold the whole K = 256, two CTAs per SM
+        CUtensorMap mh, mw;
+        if (!make_map(&mh, h[kL], Pp, kW, 128) || !make_map(&mw, Wh, kHeadPad, kW, kHeadPad))
+            return fail(NSFV1_ERR_ARGUMENT, "mlp head: tensor map encoding failed");
+        if (int st = cuda(launch_gemm<kHeadPad, 4, false, true>(mh, mw, out, (int)Pp, kHeadPad, kW, 1, kW, err, s), "mlp head")) return st;
         return cuda(cudaGetLastError(), "mlp forward");
     }
     int split_count(int64_t Pp, int tilesMN) const {
-        const int want = std::max(1, g_num_sms() / std::max(1, tilesMN));
+        const int want = std::max(1, sms / std::max(1, tilesMN));
         return (int)std::min<int64_t>(want, Pp / 64);
     }
     // backward after forward(P) and the head loss; fills grad (all entries)
@@ -529,31 +634,29 @@ struct nsfv1_mlp {
         const int64_t Pp = (P + 127) / 128 * 128;
         int used = 0;
         // head weights: C = h4^T dout -> [256 x 64]
-        if (int st = gemm(hT[kL], doutT, splitBuf, kW, kHeadPad, (int)Pp, split_count(Pp, 2), s, &used)) return st;
+        if (int st = gemm_mn(h[kL], dout, kHeadPad, (int)Pp, split_count(Pp, 2), s, &used)) return st;
         k_sum_splits_head<<<(kOut * kW + 255) / 256, 256, 0, s>>>(used, splitBuf, off, grad);
         // dh4 = dout Wh
-        if (int st = gemm(dout, WhT, dh, (int)Pp, kW, kHeadPad, 1, s)) return st;
+        if (int st = product(dout, WhT, kHeadPad, Pp, s)) return st;
         for (int l = kL - 1; l >= 0; --l) {
-            k_slot_red<<<dim3(nSlots, kRedChunks), kW, 0, s>>>(l, slotPtr, a[l], dh, prm, off, gb, part);
-            k_film_grad<<<1, kW, 0, s>>>(l, nSlots, cond, part, off, grad);
-            k_act_bwd<<<dim3((unsigned)(Pp / 32), kW / 32), dim3(32, 8), 0, s>>>(P, Pp, l, a[l], dh, prm, off, gb, pointSlot, da, daT);
+            k_act_bwd<<<(unsigned)(Pp / kBwdRows), kW / 2, 0, s>>>(P, l, a[l], dh, prm, off, gb, pointSlot, da, part + l * part_stride());
             const int in = layer_in(l);
             // dW_l = da^T h_l -> [256 x in]
-            if (int st = gemm(daT, hT[l], splitBuf, kW, in, (int)Pp, split_count(Pp, 2 * (in / std::min(in, 256))), s, &used)) return st;
+            if (int st = gemm_mn(da, h[l], in, (int)Pp, split_count(Pp, 2), s, &used)) return st;
             k_sum_splits<<<(kW * in + 255) / 256, 256, 0, s>>>(used, (int64_t)kW * in, splitBuf, grad + off.W[l]);
             // dh_l = da W_l
             if (l > 0)
-                if (int st = gemm(da, WT[l], dh, (int)Pp, in, kW, 1, s)) return st;
+                if (int st = product(da, WT[l], kW, Pp, s)) return st;
         }
+        k_slot_sum<<<dim3(nSlots, kL), kW, 0, s>>>(slotPtr, part, part_stride(), slotSum);
+        k_film_grad<<<dim3(kW / 32, kL), dim3(32, 8), 0, s>>>(nSlots, cond, slotSum, off, grad);
         return cuda(cudaGetLastError(), "mlp backward");
     }
     int head_loss(int64_t P, cudaStream_t s) {
         const int64_t Pp = (P + 127) / 128 * 128;
         const int nb = (int)((Pp + 255) / 256);
-        // rows 3..63 of the transposed output gradient are padding: zero for this row stride
-        if (int st = cuda(cudaMemsetAsync(doutT + 3 * Pp, 0, (size_t)(kHeadPad - 3) * Pp * 2, s), "mlp loss")) return st;
-        k_head_loss<<<nb, 256, 0, s>>>(P, Pp, out, prm, off, tgt, dout, doutT, lossPart, dbhPart);
-        k_head_reduce<<<1, 32, 0, s>>>(nb, P, lossPart, dbhPart, off, grad, loss);
+        k_head_loss<<<nb, 256, 0, s>>>(P, Pp, out, prm, off, tgt, dout, lossPart, dbhPart);
+        k_head_reduce<<<1, 256, 0, s>>>(nb, P, lossPart, dbhPart, off, grad, loss);
         return cuda(cudaGetLastError(), "mlp loss");
     }
     int upload_slots(int nSlots, const int32_t* slotPtrHost, cudaStream_t s) {
@@ -590,19 +693,21 @@ int nsfv1_mlp_create(const nsfv1_mlp_config* cfg, nsfv1_mlp** out) {
     al(m->prm, np * 4); al(m->grad, np * 4); al(m->am, np * 4); al(m->av, np * 4);
     for (int l = 0; l < kL; ++l) { al(m->W[l], (size_t)kW * layer_in(l) * 2); al(m->WT[l], (size_t)kW * layer_in(l) * 2); al(m->a[l], (size_t)P * kW * 4); }
     al(m->Wh, kHeadPad * kW * 2); al(m->WhT, kHeadPad * kW * 2);
-    for (int l = 0; l <= kL; ++l) { al(m->h[l], (size_t)P * layer_in(l) * 2); al(m->hT[l], (size_t)P * layer_in(l) * 2); }
-    al(m->out, (size_t)P * kHeadPad * 4); al(m->dh, (size_t)P * kW * 4);
+    for (int l = 0; l <= kL; ++l) al(m->h[l], (size_t)P * layer_in(l) * 2);
+    al(m->out, (size_t)P * kOutPad * 4); al(m->dh, (size_t)P * kW * 4);
     al(m->gb, (size_t)m->maxSlots * kL * 2 * kW * 4);
-    al(m->part, (size_t)m->maxSlots * kRedChunks * 3 * kW * 4);
-    m->splitCap = (size_t)2 * g_num_sms() * kW * kW * 4;
+    al(m->part, (size_t)kL * m->part_stride() * 4);
+    al(m->slotSum, (size_t)kL * m->maxSlots * 3 * kW * 4);
+    m->sms = g_num_sms();
+    m->splitCap = (size_t)2 * m->sms * kW * kW * 4;
     al(m->splitBuf, m->splitCap);
     al(m->cond, (size_t)m->maxSlots * 2 * 4); al(m->lid, (size_t)m->maxSlots * 4);
-    al(m->dout, (size_t)P * kHeadPad * 2); al(m->doutT, (size_t)P * kHeadPad * 2);
-    al(m->da, (size_t)P * kW * 2); al(m->daT, (size_t)P * kW * 2);
+    al(m->dout, (size_t)P * kHeadPad * 2);
+    al(m->da, (size_t)P * kW * 2);
     al(m->dbhPart, (size_t)(P / 256 + 1) * 3 * 4); al(m->lossPart, (size_t)(P / 256 + 1) * 8); al(m->loss, 8);
     al(m->tgt, (size_t)P * 3 * 4); al(m->xy, (size_t)P * 8);
     al(m->slotPtr, (size_t)(m->maxSlots + 1) * 4); al(m->pointSlot, (size_t)P * 4); al(m->err, 4);
-    if (ok) ok = cudaMemset(m->dout, 0, (size_t)P * kHeadPad * 2) == cudaSuccess && cudaMemset(m->doutT, 0, (size_t)P * kHeadPad * 2) == cudaSuccess &&
+    if (ok) ok = cudaMemset(m->dout, 0, (size_t)P * kHeadPad * 2) == cudaSuccess &&
                  cudaMemset(m->err, 0, 4) == cudaSuccess && cudaMemset(m->am, 0, np * 4) == cudaSuccess &&
                  cudaMemset(m->av, 0, np * 4) == cudaSuccess && cudaMemset(m->grad, 0, np * 4) == cudaSuccess;
     if (!ok) { delete m; return NSFV1_ERR_CUDA; }
@@ -656,7 +761,7 @@ int nsfv1_mlp_forward(nsfv1_mlp* m, int64_t n_points, const float* xy, int n_slo
     if (int st = m->upload_slots(n_slots, slot_ptr, s)) return st;
     k_film<<<dim3(n_slots, kL), kW, 0, s>>>(n_slots, m->cond, m->prm, m->off, m->gb);
     if (int st = m->cuda(cudaMemcpyAsync(m->xy, xy, n_points * 8, cudaMemcpyDeviceToDevice, s), "mlp xy")) return st;
-    if (int st = m->forward(n_points, s)) return st;
+    if (int st = m->forward(n_points, s, false)) return st;
     k_write_state<<<(unsigned)((n_points + 255) / 256), 256, 0, s>>>(n_points, 0, m->out, m->prm, m->off, m->pointSlot, nullptr, nullptr, out);
     if (int st = m->cuda(cudaGetLastError(), "mlp forward")) return st;
     return m->check_err(s);
@@ -672,7 +777,7 @@ int nsfv1_mlp_loss_grad(nsfv1_mlp* m, int64_t n_points, const float* xy, int n_s
     k_film<<<dim3(n_slots, kL), kW, 0, s>>>(n_slots, m->cond, m->prm, m->off, m->gb);
     if (int st = m->cuda(cudaMemcpyAsync(m->xy, xy, n_points * 8, cudaMemcpyDeviceToDevice, s), "mlp xy")) return st;
     if (int st = m->cuda(cudaMemcpyAsync(m->tgt, target, n_points * 12, cudaMemcpyDeviceToDevice, s), "mlp target")) return st;
-    if (int st = m->forward(n_points, s)) return st;
+    if (int st = m->forward(n_points, s, true)) return st;
     if (int st = m->head_loss(n_points, s)) return st;
     if (int st = m->backward(n_points, n_slots, s)) return st;
     if (int st = m->cuda(cudaMemcpyAsync(grad, m->grad, m->off.total * 4, cudaMemcpyDeviceToDevice, s), "mlp grad")) return st;
@@ -696,7 +801,7 @@ int nsfv1_mlp_train(nsfv1_mlp* m, const nsfv1_mlp_dataset* data, const nsfv1_mlp
         k_sample<<<(unsigned)((P + 255) / 256), 256, 0, s>>>(it + tp->step_offset, tp->seed, tp->slots, tp->points_per_slot, data->n_train,
                                                          data->n_nodes, (const float2*)data->coords, data->targets, data->cond, m->xy, m->tgt, m->cond);
         k_film<<<dim3(tp->slots, kL), kW, 0, s>>>(tp->slots, m->cond, m->prm, m->off, m->gb);
-        if (int st = m->forward(P, s)) return st;
+        if (int st = m->forward(P, s, true)) return st;
         if (int st = m->head_loss(P, s)) return st;
         if (int st = m->backward(P, tp->slots, s)) return st;
         // cosine schedule from lr to lr_final
@@ -748,7 +853,7 @@ int nsfv1_mlp_predict(nsfv1_mlp* m, int64_t n_points, const float* xy, int n_slo
         if (int st = m->upload_slots(ns, sp.data(), s)) return st;
         k_film<<<dim3(ns, kL), kW, 0, s>>>(ns, m->cond, m->prm, m->off, m->gb);
         if (int st = m->cuda(cudaMemcpyAsync(m->xy, xy + 2 * p0, P * 8, cudaMemcpyDeviceToDevice, s), "mlp xy")) return st;
-        if (int st = m->forward(P, s)) return st;
+        if (int st = m->forward(P, s, false)) return st;
         k_write_state<<<(unsigned)((P + 255) / 256), 256, 0, s>>>(P, p0, m->out, m->prm, m->off, m->pointSlot, m->lid, u, nullptr);
         if (int st = m->cuda(cudaGetLastError(), "mlp predict")) return st;
         // the staging buffers are reused by the next chunk

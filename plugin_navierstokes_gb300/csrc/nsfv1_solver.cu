@@ -402,34 +402,45 @@ __global__ void k_bicg_beta(const double* partials, int nb, double* S) {
 
 // ---- fused BiCGStab steps (FP64 Krylov vectors, Jacobian / inverse blocks of type MT) ----
 
-// sums the per-thread values v[k] of one block in a fixed tree into partials[k * gridDim.x + block]
+// the warp sums of v[k] by shuffles, then the block's warps by warp 0: valid in thread 0 (fixed tree)
+template <int K>
+__device__ __forceinline__ void block_sum(double (&v)[K]) {
+    __shared__ double sh[K][kRedThreads / 32];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], off);
+        if (lane == 0) sh[k][warp] = v[k];
+    }
+    __syncthreads();
+    if (warp == 0) {
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            v[k] = sh[k][lane & (kRedThreads / 32 - 1)];
+#pragma unroll
+            for (int off = kRedThreads / 64; off > 0; off >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], off);
+        }
+    }
+    __syncthreads();   // sh is free for a second sum
+}
+
+// sums the per-thread values v[k] of one block into partials[k * gridDim.x + block]
 template <int K>
 __device__ __forceinline__ void block_partials(double (&v)[K], double* __restrict__ partials) {
-    __shared__ double sh[K][kRedThreads];
-#pragma unroll
-    for (int k = 0; k < K; ++k) sh[k][threadIdx.x] = v[k];
-    __syncthreads();
-    for (int st = kRedThreads / 2; st > 0; st >>= 1) {
-        if (threadIdx.x < st) {
-#pragma unroll
-            for (int k = 0; k < K; ++k) sh[k][threadIdx.x] += sh[k][threadIdx.x + st];
-        }
-        __syncthreads();
-    }
+    block_sum<K>(v);
     if (threadIdx.x == 0) {
 #pragma unroll
-        for (int k = 0; k < K; ++k) partials[k * gridDim.x + blockIdx.x] = sh[k][0];
+        for (int k = 0; k < K; ++k) partials[k * gridDim.x + blockIdx.x] = v[k];
     }
 }
 
 // After block_partials<K>: the block that finishes last (counted in *counter)
-// sums the partials of all blocks, in block order (the sums of block_sum_partials),
-// into out (valid in thread 0) and returns true; the counter is left at 0.
-// Partials are read past L1 (other SMs wrote them).
+// sums the partials of all blocks in a fixed order into out (valid in thread 0) and returns
+// true; the counter is left at 0. Partials are read past L1 (other SMs wrote them).
 template <int K>
 __device__ __forceinline__ bool last_block_sum(const double* __restrict__ partials, unsigned* counter, double (&out)[K]) {
     __shared__ bool amLast;
-    __shared__ double sh[K][kRedThreads];
     if (threadIdx.x == 0) {
         __threadfence();
         amLast = atomicAdd(counter, 1u) == gridDim.x - 1;
@@ -437,29 +448,43 @@ __device__ __forceinline__ bool last_block_sum(const double* __restrict__ partia
     __syncthreads();
     if (!amLast) return false;
     __threadfence();
+    constexpr int U = (kRedBlocks + kRedThreads - 1) / kRedThreads;
     const int nb = gridDim.x;
-    double acc[K];
+    double p[K][U];
 #pragma unroll
-    for (int k = 0; k < K; ++k) acc[k] = 0.0;
-    for (int i = threadIdx.x; i < nb; i += kRedThreads)
+    for (int k = 0; k < K; ++k)
 #pragma unroll
-        for (int k = 0; k < K; ++k) acc[k] += __ldcg(partials + k * nb + i);
-#pragma unroll
-    for (int k = 0; k < K; ++k) sh[k][threadIdx.x] = acc[k];
-    __syncthreads();
-    for (int st = kRedThreads / 2; st > 0; st >>= 1) {
-        if (threadIdx.x < st) {
-#pragma unroll
-            for (int k = 0; k < K; ++k) sh[k][threadIdx.x] += sh[k][threadIdx.x + st];
+        for (int i = 0; i < U; ++i) {
+            const int q = threadIdx.x + i * kRedThreads;
+            p[k][i] = q < nb ? __ldcg(partials + k * nb + q) : 0.0;
         }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
 #pragma unroll
-        for (int k = 0; k < K; ++k) out[k] = sh[k][0];
-        *counter = 0u;
+    for (int k = 0; k < K; ++k) {
+        out[k] = p[k][0];
+#pragma unroll
+        for (int i = 1; i < U; ++i) out[k] += p[k][i];
     }
+    block_sum<K>(out);
+    if (threadIdx.x == 0) *counter = 0u;
     return true;
+}
+
+// f(i) for the entries of this thread in a grid-stride walk, the loads of four entries in flight:
+// load(i, slot) fetches, use(slot) consumes in order
+template <class Load, class Use>
+__device__ __forceinline__ void strided4(const int64_t n, Load&& load, Use&& use) {
+    const int64_t step = (int64_t)gridDim.x * kRedThreads;
+    int64_t i = (int64_t)blockIdx.x * kRedThreads + threadIdx.x;
+    for (; i + 3 * step < n; i += 4 * step) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) load(i + k * step, k);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) use(i + k * step, k);
+    }
+    for (; i < n; i += step) {
+        load(i, 0);
+        use(i, 0);
+    }
 }
 
 // out = Dinv_row x (the point-block Jacobi apply of k_prec, same summation)
@@ -548,7 +573,7 @@ __global__ void k_bicg_s_prec(int64_t nRows, const double* __restrict__ S, const
 }
 
 // x += alpha ph + omega sh; r = s - omega t; partials of (r, r) and (r0, r)
-// (the grid-stride layout of k_dot_partial, kRedBlocks blocks)
+// (a grid-stride walk, kRedBlocks blocks)
 
 // the scalar updates that follow the reductions (thread 0 of the last block)
 __device__ __forceinline__ void bicg_alpha_update(double* S, const double r0v) {
@@ -563,13 +588,12 @@ __device__ __forceinline__ void bicg_omega_update(double* S, const double ts, co
     S[S_OMEGA] = isfinite(omega) ? omega : 0.0;
 }
 
-// (r0, v) and alpha in one launch (k_dot_partial's grid and tree, then the last block)
+// (r0, v) and alpha in one launch
 __global__ void __launch_bounds__(kRedThreads) k_bicg_dot_alpha(int64_t n, const double* __restrict__ r0, const double* __restrict__ v,
                                                                  double* __restrict__ partials, unsigned* counter, double* S) {
     if (S[S_DONE] != 0.0) return;
-    double d[1] = {0.0};
-    for (int64_t i = (int64_t)blockIdx.x * kRedThreads + threadIdx.x; i < n; i += (int64_t)gridDim.x * kRedThreads)
-        d[0] += r0[i] * v[i];
+    double d[1] = {0.0}, a[4], c[4];
+    strided4(n, [&](int64_t i, int k) { a[k] = r0[i]; c[k] = v[i]; }, [&](int64_t, int k) { d[0] += a[k] * c[k]; });
     block_partials<1>(d, partials);
     double tot[1];
     if (last_block_sum<1>(partials, counter, tot) && threadIdx.x == 0) bicg_alpha_update(S, tot[0]);
@@ -579,12 +603,12 @@ __global__ void __launch_bounds__(kRedThreads) k_bicg_dot_alpha(int64_t n, const
 __global__ void __launch_bounds__(kRedThreads) k_bicg_dot_omega(int64_t n, const double* __restrict__ t, const double* __restrict__ sv,
                                                                  double* __restrict__ partials, unsigned* counter, double* S) {
     if (S[S_DONE] != 0.0) return;
-    double d[2] = {0.0, 0.0};
-    for (int64_t i = (int64_t)blockIdx.x * kRedThreads + threadIdx.x; i < n; i += (int64_t)gridDim.x * kRedThreads) {
-        const double ti = t[i];
-        d[0] += ti * sv[i];
-        d[1] += ti * ti;
-    }
+    double d[2] = {0.0, 0.0}, a[4], c[4];
+    strided4(n, [&](int64_t i, int k) { a[k] = t[i]; c[k] = sv[i]; },
+             [&](int64_t, int k) {
+                 d[0] += a[k] * c[k];
+                 d[1] += a[k] * a[k];
+             });
     block_partials<2>(d, partials);
     double tot[2];
     if (last_block_sum<2>(partials, counter, tot) && threadIdx.x == 0) bicg_omega_update(S, tot[0], tot[1]);
@@ -616,14 +640,15 @@ __global__ void __launch_bounds__(kRedThreads) k_bicg_x_end(int64_t n, double* S
                                                              unsigned* counter, double nr0, double rtol) {
     if (S[S_DONE] != 0.0) return;
     const double alpha = S[S_ALPHA], omega = S[S_OMEGA];
-    double d[2] = {0.0, 0.0};
-    for (int64_t i = (int64_t)blockIdx.x * kRedThreads + threadIdx.x; i < n; i += (int64_t)gridDim.x * kRedThreads) {
-        x[i] += alpha * ph[i] + omega * shv[i];
-        const double ri = sv[i] - omega * t[i];
-        r[i] = ri;
-        d[0] += ri * ri;
-        d[1] += r0[i] * ri;
-    }
+    double d[2] = {0.0, 0.0}, xi[4], pi[4], hi[4], si[4], ti[4], qi[4];
+    strided4(n, [&](int64_t i, int k) { xi[k] = x[i]; pi[k] = ph[i]; hi[k] = shv[i]; si[k] = sv[i]; ti[k] = t[i]; qi[k] = r0[i]; },
+             [&](int64_t i, int k) {
+                 x[i] = xi[k] + (alpha * pi[k] + omega * hi[k]);
+                 const double ri = si[k] - omega * ti[k];
+                 r[i] = ri;
+                 d[0] += ri * ri;
+                 d[1] += qi[k] * ri;
+             });
     block_partials<2>(d, partials);
     double tot[2];
     if (last_block_sum<2>(partials, counter, tot) && threadIdx.x == 0) bicg_end_update(S, tot, nr0, rtol);
@@ -1069,6 +1094,15 @@ static cudaError_t spmv(const Disc& D, const MT* vals, const VT* x, VT* y, cudaS
     return cudaGetLastError();
 }
 
+// y = A x for an FP32 matrix and split x
+static cudaError_t spmv_split(const Disc& D, const float* vals, const float2* xs, double* y, cudaStream_t s, const double* gate = nullptr) {
+    const int64_t nR = D.nNodes;
+    constexpr int G4 = spmv_lanes<4>(), G3 = spmv_lanes<3>();
+    if (D.dim == 3) k_bsr_mv_split<4, G4><<<grid_for(nR * G4), 256, 0, s>>>(nR, D.d_rowPtr, D.d_colIdx, vals, xs, y, gate);
+    else k_bsr_mv_split<3, G3><<<grid_for(nR * G3), 256, 0, s>>>(nR, D.d_rowPtr, D.d_colIdx, vals, xs, y, gate);
+    return cudaGetLastError();
+}
+
 template <typename VT, int K>
 static void dots(int64_t n, const VT* const (&a)[K], const VT* const (&c)[K], double* partials, cudaStream_t s,
                  const double* gate = nullptr) {
@@ -1149,8 +1183,7 @@ static void bicg_iteration(Disc& D, const MT* J, const MT* Dinv, double* const (
     const int gn = grid_for(nR);
     auto mv = [&](const double* xd, const float2* xsplit, double* y) {
         if constexpr (std::is_same<MT, float>::value) {
-            constexpr int G = spmv_lanes<b>();
-            k_bsr_mv_split<b, G><<<grid_for(nR * G), 256, 0, s>>>(nR, D.d_rowPtr, D.d_colIdx, J, xsplit, y, done);
+            spmv_split(D, J, xsplit, y, s, done);
         } else {
             spmv<MT, double>(D, J, xd, y, s, done);
         }
@@ -1490,16 +1523,8 @@ int nsfv1_bsr_mv_split(nsfv1_disc* h, const float* vals, const float* xs, double
     if (!D->hasMesh) { D->fail(NSFV1_ERR_STATE, "bsr_mv_split: no mesh"); return D->status; }
     if (!vals || !xs || !y) { D->fail(NSFV1_ERR_ARGUMENT, "bsr_mv_split: null pointer"); return D->status; }
     if (reinterpret_cast<uintptr_t>(xs) & 7) { D->fail(NSFV1_ERR_ARGUMENT, "bsr_mv_split: xs must be 8-byte aligned"); return D->status; }
-    const int64_t nR = D->nNodes;
     cudaStream_t s = (cudaStream_t)stream;
-    const float2* x2 = reinterpret_cast<const float2*>(xs);
-    if (D->dim == 3) {
-        constexpr int G = spmv_lanes<4>();
-        k_bsr_mv_split<4, G><<<grid_for(nR * G), 256, 0, s>>>(nR, D->d_rowPtr, D->d_colIdx, vals, x2, y, nullptr);
-    } else {
-        constexpr int G = spmv_lanes<3>();
-        k_bsr_mv_split<3, G><<<grid_for(nR * G), 256, 0, s>>>(nR, D->d_rowPtr, D->d_colIdx, vals, x2, y, nullptr);
-    }
+    if (!D->cuda_ok(spmv_split(*D, vals, reinterpret_cast<const float2*>(xs), y, s), "bsr_mv_split")) return D->status;
     return D->cuda_ok(cudaGetLastError(), "bsr_mv_split") ? NSFV1_OK : D->status;
 }
 

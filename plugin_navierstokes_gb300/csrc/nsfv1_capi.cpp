@@ -85,9 +85,56 @@ void Disc::free_mesh() {
     outflowHost.clear();
     bndFluxHost.clear();
     dfree(d_instNode0); dfree(d_elemInst); dfree(d_nodeInst); dfree(d_instActive);
+    dfree(d_diagPtr); dfree(d_diagSlot); dfree(d_diagStage);
     nInst = 0; instNode0.clear(); instSkip = false;
     // the batched solver's levels, graphs and buffers belong to this mesh
     if (batch) { batch_free(batch); batch = nullptr; }
+}
+
+// Staging of the one-launch FP32 Jacobian of a 2D mesh: slot of every (element, corner), a node's
+// slots in the colour order of its elements. Not an error where it cannot be had (an edge in
+// three elements, no memory for the stage): the mesh is then assembled colour by colour.
+bool Disc::setup_diag_stage(const std::vector<int32_t>& nodeElemPtr) {
+    dfree(d_diagPtr); dfree(d_diagSlot); dfree(d_diagStage);
+    if (dim != 2) return true;
+    // on the device, where the mesh is already: a few launches (the host loops took a sixth of set_mesh)
+    int32_t *tmp = nullptr, *d_ptr = nullptr, *d_slot = nullptr;
+    float* d_stage = nullptr;
+    const size_t nTmp = std::max(colIdx.size(), (size_t)nNodes) + 1;
+    bool ok = cudaMalloc((void**)&tmp, nTmp * sizeof(int32_t)) == cudaSuccess && dupload(d_ptr, nodeElemPtr.data(), nodeElemPtr.size()) == cudaSuccess;
+    int many = 1;
+    if (ok) ok = launch_count_blocks(nsh, nElems, d_elemBlk, (int64_t)colIdx.size(), tmp, nullptr) == cudaSuccess &&
+                 cudaMemcpy(&many, tmp + colIdx.size(), sizeof(int), cudaMemcpyDeviceToHost) == cudaSuccess;
+    if (ok && !many) {
+        ok = cudaMalloc((void**)&d_slot, (size_t)nElems * nsh * sizeof(int32_t)) == cudaSuccess &&
+             cudaMalloc((void**)&d_stage, (size_t)nElems * nsh * 9 * sizeof(float)) == cudaSuccess &&
+             cudaMemset(tmp, 0, (size_t)nNodes * sizeof(int32_t)) == cudaSuccess;
+        for (int c = 0; ok && c < nColors; ++c)
+            ok = launch_assign_slots(nsh, d_colorElems + colorPtr[c], colorPtr[c + 1] - colorPtr[c], d_conn, d_ptr, tmp, d_slot, nullptr) == cudaSuccess;
+        if (ok) ok = cudaStreamSynchronize(nullptr) == cudaSuccess;
+    }
+    dfree(tmp);
+    if (ok && !many) {
+        d_diagPtr = d_ptr; d_diagSlot = d_slot; d_diagStage = d_stage;
+    } else {
+        cudaGetLastError();
+        dfree(d_ptr); dfree(d_slot); dfree(d_stage);
+    }
+    return true;
+}
+
+// The FP32 Jacobian of all elements in one launch where that is served (it skips no instance);
+// the values are cleared already
+bool Disc::jacobian_f32_at_once(const DiscParams& P, const AsmArgs& whole, cudaStream_t s, bool& served) {
+    served = d_diagStage && !instSkip && !uses_ipshape(P);
+    if (!served) return true;
+    AsmArgs a = whole;
+    a.elems = nullptr;
+    a.count = (int32_t)nElems;
+    a.diagSlot = d_diagSlot;
+    a.diagStage = d_diagStage;
+    return cuda_ok(launch_jacobian_lanes(roid, P, a, s), "jacobian kernel") &&
+           cuda_ok(launch_diag_sum(dim + 1, nNodes, d_diagPtr, d_diagStage, d_diagPos, (float*)a.vals, s), "diagonal blocks");
 }
 
 void Disc::free_outflow() {
@@ -192,11 +239,12 @@ bool Disc::check_err_word(cudaStream_t s) {
 
 // block-CSR pattern: every node pair sharing an element, columns sorted
 static void build_pattern(int nsh, int64_t nNodes, int64_t nElems, const int32_t* conn, std::vector<int32_t>& rowPtr,
-                          std::vector<int32_t>& colIdx, std::vector<int32_t>& elemBlk) {
+                          std::vector<int32_t>& colIdx, std::vector<int32_t>& elemBlk, std::vector<int32_t>* nodeElemPtr = nullptr) {
     // node -> incident elements
     std::vector<int64_t> nptr(nNodes + 1, 0);
     for (int64_t k = 0; k < nElems * nsh; ++k) nptr[conn[k] + 1]++;
     for (int64_t r = 0; r < nNodes; ++r) nptr[r + 1] += nptr[r];
+    if (nodeElemPtr) nodeElemPtr->assign(nptr.begin(), nptr.end());
     std::vector<int32_t> nel(nptr[nNodes]);
     {
         std::vector<int64_t> fill(nptr.begin(), nptr.end() - 1);
@@ -427,7 +475,8 @@ int nsfv1_set_mesh(nsfv1_disc* h, int elem_type, int64_t n_nodes, const double* 
         D->coordsHost.assign(coords, coords + n_nodes * dim);
         D->connHost.assign(conn, conn + n_elems * nsh);
         D->nuElemHost.clear(); D->dirRowHost.clear(); D->dirValHost.clear(); D->instCells.clear();
-        build_pattern(nsh, n_nodes, n_elems, conn, D->rowPtr, D->colIdx, D->elemBlk);
+        std::vector<int32_t> nodeElemPtr;
+        build_pattern(nsh, n_nodes, n_elems, conn, D->rowPtr, D->colIdx, D->elemBlk, dim == 2 ? &nodeElemPtr : nullptr);
         D->nColors = build_coloring(nsh, n_nodes, n_elems, conn, D->color);
         if (D->nColors < 0) { D->fail(NSFV1_ERR_ARGUMENT, "too many element colours"); return D->status; }
         D->colorPtr.assign(D->nColors + 1, 0);
@@ -464,7 +513,7 @@ int nsfv1_set_mesh(nsfv1_disc* h, int elem_type, int64_t n_nodes, const double* 
             if (!D->cuda_ok(cudaMalloc((void**)&D->d_err, sizeof(int)), "alloc err")) return D->status;
         }
         if (!D->cuda_ok(cudaMemset(D->d_err, 0, sizeof(int)), "memset err")) return D->status;
-        if (!D->ensure_ipws()) return D->status;
+        if (!D->ensure_ipws() || !D->setup_diag_stage(nodeElemPtr)) return D->status;
         D->nDir = 0;
         D->free_workspace();
         D->hasMesh = true;
@@ -1032,7 +1081,7 @@ bool Disc::assemble_defect(const double* u, const double* u_old, double dt, doub
     if (!cuda_ok(cudaMemsetAsync(d, 0, sizeof(double) * nNodes * b, s), "memset defect")) return false;
     for (int c = 0; c < nColors; ++c) {
         AsmArgs a{d_coords, d_conn, d_elemBlk, d_colorElems + colorPtr[c], colorPtr[c + 1] - colorPtr[c], d_err, u, u_old, d, nullptr,
-                  d_nuElem, instSkip ? d_elemInst : nullptr, d_instActive, nNodes, (int64_t)colIdx.size(), colorAffine[c]};
+                  d_nuElem, instSkip ? d_elemInst : nullptr, d_instActive, nNodes, (int64_t)colIdx.size(), nullptr, nullptr, colorAffine[c]};
         if (!cuda_ok(launch_defect(roid, P, a, s, asmThreads), "defect kernel")) return false;
     }
     if (!outflow_terms(P, u, d, nullptr, 0, s)) return false;
@@ -1053,10 +1102,16 @@ bool Disc::assemble_defect_jacobian(const double* u, const double* u_old, double
     if (!cuda_ok(cudaMemsetAsync(d, 0, sizeof(double) * nNodes * b, s), "memset defect")) return false;
     const size_t vsize = prec == NSFV1_F64 ? sizeof(double) : sizeof(float);
     if (!cuda_ok(cudaMemsetAsync(vals, 0, colIdx.size() * b * b * vsize, s), "memset jacobian")) return false;
+    bool jacDone = false;
+    if (prec == NSFV1_F32) {
+        const AsmArgs whole{d_coords, d_conn, d_elemBlk, nullptr, 0, d_err, u, u_old, nullptr, vals, d_nuElem, nullptr, d_instActive, nNodes, (int64_t)colIdx.size()};
+        if (!jacobian_f32_at_once(P, whole, s, jacDone)) return false;
+    }
     for (int c = 0; c < nColors; ++c) {
         AsmArgs a{d_coords, d_conn, d_elemBlk, d_colorElems + colorPtr[c], colorPtr[c + 1] - colorPtr[c], d_err, u, u_old, d, vals,
-                  d_nuElem, instSkip ? d_elemInst : nullptr, d_instActive, nNodes, (int64_t)colIdx.size(), colorAffine[c]};
-        if (!cuda_ok(launch_defect_jacobian(roid, P, a, prec, s, asmThreads), "defect+jacobian kernel")) return false;
+                  d_nuElem, instSkip ? d_elemInst : nullptr, d_instActive, nNodes, (int64_t)colIdx.size(), nullptr, nullptr, colorAffine[c]};
+        if (!cuda_ok(jacDone ? launch_defect(roid, P, a, s, asmThreads) : launch_defect_jacobian(roid, P, a, prec, s, asmThreads), "defect+jacobian kernel"))
+            return false;
     }
     if (!outflow_terms(P, u, d, vals, prec, s)) return false;
     if (!cuda_ok(launch_bnd_flux(b, nNodes, u_old ? dt : 1.0, d_bndFlux, d, s), "inflow flux")) return false;
@@ -1075,9 +1130,14 @@ bool Disc::assemble_jacobian(const double* u, const double* u_old, double dt, vo
     const int b = dim + 1;
     const size_t bytes = colIdx.size() * b * b * (prec == NSFV1_F64 ? sizeof(double) : sizeof(float));
     if (!cuda_ok(cudaMemsetAsync(vals, 0, bytes, s), "memset jacobian")) return false;
-    for (int c = 0; c < nColors; ++c) {
+    bool jacDone = false;
+    if (prec == NSFV1_F32) {
+        const AsmArgs whole{d_coords, d_conn, d_elemBlk, nullptr, 0, d_err, u, u_old, nullptr, vals, d_nuElem, nullptr, d_instActive, nNodes, (int64_t)colIdx.size()};
+        if (!jacobian_f32_at_once(P, whole, s, jacDone)) return false;
+    }
+    for (int c = 0; c < (jacDone ? 0 : nColors); ++c) {
         AsmArgs a{d_coords, d_conn, d_elemBlk, d_colorElems + colorPtr[c], colorPtr[c + 1] - colorPtr[c], d_err, u, u_old, nullptr, vals,
-                  d_nuElem, instSkip ? d_elemInst : nullptr, d_instActive, nNodes, (int64_t)colIdx.size(), colorAffine[c]};
+                  d_nuElem, instSkip ? d_elemInst : nullptr, d_instActive, nNodes, (int64_t)colIdx.size(), nullptr, nullptr, colorAffine[c]};
         if (!cuda_ok(launch_jacobian(roid, P, a, prec, s, asmThreads), "jacobian kernel")) return false;
     }
     if (!outflow_terms(P, u, nullptr, vals, prec, s)) return false;

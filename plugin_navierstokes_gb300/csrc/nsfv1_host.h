@@ -26,6 +26,8 @@ struct Workspace {
     double* hscal = nullptr;  // pinned host mirror of the scalars
 };
 
+struct AsmArgs;
+
 struct Disc {
     int dim = 2;
     // parameters (defaults of the reference constructors)
@@ -44,6 +46,10 @@ struct Disc {
     std::vector<int32_t> colorAffine;   // affine elements of each colour: they come first in its part of colorElems
     double* d_coords = nullptr;
     int32_t *d_conn = nullptr, *d_elemBlk = nullptr, *d_colorElems = nullptr, *d_rowPtr = nullptr, *d_colIdx = nullptr;
+    // 2D meshes whose off-diagonal blocks get at most two contributions: the staged diagonal blocks
+    // of the one-launch FP32 Jacobian (nsfv1_jac_lanes.cu); null where it is not served
+    int32_t *d_diagPtr = nullptr, *d_diagSlot = nullptr;
+    float* d_diagStage = nullptr;
     int32_t* d_diagPos = nullptr;   // block index of each row's diagonal block
     double* d_nuElem = nullptr;     // per-element viscosity (nsfv1_set_elem_viscosity), or null
     // independent instances (nsfv1_set_instances): node ranges, element -> instance
@@ -102,6 +108,8 @@ struct Disc {
     bool assemble_jacobian(const double* u, const double* u_old, double dt, void* vals, int prec, cudaStream_t s, bool sync = true);
     bool assemble_defect_jacobian(const double* u, const double* u_old, double dt, double* d, void* vals, int prec, cudaStream_t s);
     bool ensure_workspace(int prec, int gmresM);
+    bool setup_diag_stage(const std::vector<int32_t>& nodeElemPtr);   // [nNodes + 1] offsets of the elements around a node
+    bool jacobian_f32_at_once(const DiscParams& P, const AsmArgs& whole, cudaStream_t s, bool& served);
     bool set_dirichlet_values(double* u, cudaStream_t s);   // u[dof] = g for every Dirichlet row
 };
 

@@ -25,6 +25,10 @@ struct AsmArgs {
     const int32_t* instActive;// per-instance flag: elements of inactive instances are skipped
     int64_t nNodes = 0;       // index bounds checked by a build with NSFV1_BOUNDS_CHECK
     int64_t nnzb = 0;
+    // FP32 Jacobian of a whole 2D mesh in one launch (elems null: element t is t): the elements'
+    // diagonal blocks go to diagStage[diagSlot[e][corner]] and are summed by launch_diag_sum
+    const int32_t* diagSlot = nullptr;
+    float* diagStage = nullptr;
     int32_t nAffine = 0;      // elems[0, nAffine) have an affine reference mapping (elem_is_affine)
 };
 
@@ -47,6 +51,13 @@ cudaError_t launch_defect_jacobian(int roid, const DiscParams& P, const AsmArgs&
 cudaError_t launch_elem_batch(int roid, const DiscParams& P, const ElemBatchArgs& a, cudaStream_t s);
 // FP32 Jacobian (values only, no defect) with one lane per element corner
 cudaError_t launch_jacobian_lanes(int roid, const DiscParams& P, const AsmArgs& a, cudaStream_t s);
+// set-up of the staged diagonal blocks: contributions per off-diagonal block in count[nnzb], and
+// count[nnzb] = 1 if some block has more than two; the slots of one colour's elements
+cudaError_t launch_count_blocks(int nsh, int64_t nElems, const int32_t* elemBlk, int64_t nnzb, int32_t* count, cudaStream_t s);
+cudaError_t launch_assign_slots(int nsh, const int32_t* elems, int32_t count, const int32_t* conn, const int32_t* ptr, int32_t* fill, int32_t* slot,
+                                cudaStream_t s);
+// vals[diagPos[node]] = sum of the node's staged diagonal blocks in order (b x b FP32)
+cudaError_t launch_diag_sum(int b, int64_t nNodes, const int32_t* diagPtr, const float* stage, const int32_t* diagPos, float* vals, cudaStream_t s);
 // The positive-upwind element path (uses_ipshape(P)): defect, Jacobian (prec 0: FP64,
 // 1: FP32 values of FP64 arithmetic) and the stiffness part of the element batch;
 // P.ipws must hold ipws_doubles_host(dim) doubles for each of P.ipwsStride threads.

@@ -85,7 +85,8 @@ void Disc::free_mesh() {
     outflowHost.clear();
     bndFluxHost.clear();
     dfree(d_instNode0); dfree(d_elemInst); dfree(d_nodeInst); dfree(d_instActive);
-    dfree(d_diagPtr); dfree(d_diagSlot); dfree(d_diagStage);
+    dfree(d_diagPtr);
+    d_diagSlot = nullptr; d_diagStage = nullptr;
     nInst = 0; instNode0.clear(); instSkip = false;
     // the batched solver's levels, graphs and buffers belong to this mesh
     if (batch) { batch_free(batch); batch = nullptr; }
@@ -95,30 +96,31 @@ void Disc::free_mesh() {
 // slots in the colour order of its elements. Not an error where it cannot be had (an edge in
 // three elements, no memory for the stage): the mesh is then assembled colour by colour.
 bool Disc::setup_diag_stage(const std::vector<int32_t>& nodeElemPtr) {
-    dfree(d_diagPtr); dfree(d_diagSlot); dfree(d_diagStage);
+    dfree(d_diagPtr);
+    d_diagSlot = nullptr; d_diagStage = nullptr;
     if (dim != 2) return true;
-    // on the device, where the mesh is already: a few launches (the host loops took a sixth of set_mesh)
-    int32_t *tmp = nullptr, *d_ptr = nullptr, *d_slot = nullptr;
-    float* d_stage = nullptr;
-    const size_t nTmp = std::max(colIdx.size(), (size_t)nNodes) + 1;
-    bool ok = cudaMalloc((void**)&tmp, nTmp * sizeof(int32_t)) == cudaSuccess && dupload(d_ptr, nodeElemPtr.data(), nodeElemPtr.size()) == cudaSuccess;
+    // on the device, where the mesh is already (host loops took a sixth of set_mesh); one allocation:
+    // offsets, slots, stage, and the stage holds the counters meanwhile
+    const size_t nPtr = ((size_t)nNodes + 1 + 3) / 4 * 4, nSlot = ((size_t)nElems * nsh + 3) / 4 * 4;
+    const size_t nStage = std::max((size_t)nElems * nsh * 9, std::max(colIdx.size(), (size_t)nNodes) + 1);
+    int32_t* buf = nullptr;
+    if (cudaMalloc((void**)&buf, (nPtr + nSlot + nStage) * sizeof(int32_t)) != cudaSuccess) { cudaGetLastError(); return true; }
+    int32_t *ptr = buf, *slot = buf + nPtr, *tmp = slot + nSlot;
     int many = 1;
-    if (ok) ok = launch_count_blocks(nsh, nElems, d_elemBlk, (int64_t)colIdx.size(), tmp, nullptr) == cudaSuccess &&
-                 cudaMemcpy(&many, tmp + colIdx.size(), sizeof(int), cudaMemcpyDeviceToHost) == cudaSuccess;
+    bool ok = launch_count_blocks(nsh, nElems, d_elemBlk, (int64_t)colIdx.size(), tmp, nullptr) == cudaSuccess &&
+              cudaMemcpy(&many, tmp + colIdx.size(), sizeof(int), cudaMemcpyDeviceToHost) == cudaSuccess;
     if (ok && !many) {
-        ok = cudaMalloc((void**)&d_slot, (size_t)nElems * nsh * sizeof(int32_t)) == cudaSuccess &&
-             cudaMalloc((void**)&d_stage, (size_t)nElems * nsh * 9 * sizeof(float)) == cudaSuccess &&
+        ok = cudaMemcpy(ptr, nodeElemPtr.data(), nodeElemPtr.size() * sizeof(int32_t), cudaMemcpyHostToDevice) == cudaSuccess &&
              cudaMemset(tmp, 0, (size_t)nNodes * sizeof(int32_t)) == cudaSuccess;
         for (int c = 0; ok && c < nColors; ++c)
-            ok = launch_assign_slots(nsh, d_colorElems + colorPtr[c], colorPtr[c + 1] - colorPtr[c], d_conn, d_ptr, tmp, d_slot, nullptr) == cudaSuccess;
+            ok = launch_assign_slots(nsh, d_colorElems + colorPtr[c], colorPtr[c + 1] - colorPtr[c], d_conn, ptr, tmp, slot, nullptr) == cudaSuccess;
         if (ok) ok = cudaStreamSynchronize(nullptr) == cudaSuccess;
     }
-    dfree(tmp);
     if (ok && !many) {
-        d_diagPtr = d_ptr; d_diagSlot = d_slot; d_diagStage = d_stage;
+        d_diagPtr = ptr; d_diagSlot = slot; d_diagStage = reinterpret_cast<float*>(tmp);
     } else {
         cudaGetLastError();
-        dfree(d_ptr); dfree(d_slot); dfree(d_stage);
+        cudaFree(buf);
     }
     return true;
 }

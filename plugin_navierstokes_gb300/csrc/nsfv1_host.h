@@ -47,7 +47,8 @@ struct Disc {
     double* d_coords = nullptr;
     int32_t *d_conn = nullptr, *d_elemBlk = nullptr, *d_colorElems = nullptr, *d_rowPtr = nullptr, *d_colIdx = nullptr;
     // 2D meshes whose off-diagonal blocks get at most two contributions: the staged diagonal blocks
-    // of the one-launch FP32 Jacobian (nsfv1_jac_lanes.cu); null where it is not served
+    // of the one-launch FP32 Jacobian (nsfv1_jac_lanes.cu), one allocation owned by d_diagPtr; null
+    // where it is not served
     int32_t *d_diagPtr = nullptr, *d_diagSlot = nullptr;
     float* d_diagStage = nullptr;
     int32_t* d_diagPos = nullptr;   // block index of each row's diagonal block

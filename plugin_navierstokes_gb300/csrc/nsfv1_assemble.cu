@@ -338,11 +338,21 @@ static cudaError_t launch_fast(int roid, const DiscParams& P, const AsmArgs& a, 
     }
     auto part = [&](auto dim, auto flow, auto affine, const AsmArgs& q) {
         constexpr int DIM = decltype(dim)::value;
-        using TN = Ten<DIM>;
         if (q.count <= 0) return;
-        const int per = t / 32 * TN::EPW, grid = (q.count + per - 1) / per;
-        k_tensor<DIM, JAC, decltype(flow)::value, decltype(affine)::value>
-            <<<grid, t, (size_t)TN::warp_doubles(JAC) * (t / 32) * sizeof(double), s>>>(P, q);
+        auto go = [&](auto split) {
+            constexpr bool SP = decltype(split)::value;
+            using TN = Ten<DIM, SP>;
+            const int per = t / 32 * TN::EPW, grid = (q.count + per - 1) / per;
+            k_tensor<DIM, JAC, decltype(flow)::value, decltype(affine)::value, SP>
+                <<<grid, t, (size_t)TN::warp_doubles(JAC) * (t / 32) * sizeof(double), s>>>(P, q);
+        };
+        // a lane per SCVF while its warps still find a sub-partition each (4 x 152): the launch then takes
+        // one SCVF's chain instead of two (32^2 cells, defect + Jacobian: 143 -> 118 us); with more
+        // elements the shared geometry of a lane's two SCVFs counts more
+        if constexpr (DIM == 2) {
+            if (q.count <= 4 * 152 * Ten<2, true>::EPW) { go(std::true_type{}); return; }
+        }
+        go(std::false_type{});
     };
     auto both = [&](auto affine, const AsmArgs& q) {
         const bool flow = P.stab == STAB_FLOW;

@@ -28,8 +28,8 @@
 //    matrix by consecutive entries.
 // Counted per hexahedron: 7.7 k FP64 instructions for LPS + FLOW defect and Jacobian (13.2 k
 // before), with the FP64 pipe 78 % active (its practical limit is 16/19). Measured, one thread
-// per element before -> here: 64^3 affine, defect + Jacobian 7.75 -> 4.43 ms; 41^3 distorted
-// transient, defect 2.56 -> 0.92 ms; 32^2 quadrilaterals 293 -> 141 us. With 8-byte reductions
+// per element before -> here: 64^3 affine, defect + Jacobian 7.73 -> 4.47 ms; 41^3 distorted
+// transient, defect 2.56 -> 0.92 ms; 32^2 quadrilaterals 293 -> 118 us (143 without SPLIT). With 8-byte reductions
 // straight from the lanes the first was 5.6 ms (138 G sectors/s into L2).
 //
 // Determinism: the SCVFs of one direction touch disjoint rows, and __syncwarp
@@ -48,9 +48,11 @@ inline bool plain_params(const DiscParams& P, const bool jac) {
            (P.convUpwind == UPW_NO || P.convUpwind == UPW_FULL || P.convUpwind == UPW_LPS);
 }
 
-template <int DIM>
+template <int DIM, bool SPLIT = false>
 struct Ten {
-    static constexpr int NSH = 1 << DIM, L = NSH / 2, B = DIM + 1, EPW = 32 / L, NQ = NSH / 2;
+    static_assert(DIM == 2 || !SPLIT, "a lane per SCVF for quadrilaterals only");
+    static constexpr int NSH = 1 << DIM, L = SPLIT ? NSH : NSH / 2, B = DIM + 1, EPW = 32 / L;
+    static constexpr int CPL = NSH / L;   // corners that a lane loads
     // corner with bits (x, y, z) in the reference element's order
     static __device__ __forceinline__ int corner(const int bits) {
         const int x = bits & 1, y = (bits >> 1) & 1;
@@ -175,10 +177,13 @@ __device__ __forceinline__ void ten_exit(const double (&t)[DIM], const int e, co
 // One colour's elements [0, count) of A.elems, all affine or (AFFINE = false) any; LPS only
 // with AFFINE. JAC: the Jacobian, and the defect if A.D is set; else the defect alone.
 // FLOW: the FLOW stabilisation, else FIELDS.
-template <int DIM, bool JAC, bool FLOW, bool AFFINE>
-__global__ void __launch_bounds__(kThreads, 3) k_tensor(const DiscParams P, const AsmArgs A) {
-    using T = Ten<DIM>;
-    constexpr int NSH = T::NSH, L = T::L, B = T::B, EPW = T::EPW, Pc = DIM;
+// SPLIT (quadrilaterals): a lane per SCVF instead of one per position with both directions, for
+// launches of few warps, whose time is a lane's serial chain. Lanes of the two directions meet
+// in the same rows; their reductions take turns.
+template <int DIM, bool JAC, bool FLOW, bool AFFINE, bool SPLIT = false>
+__global__ void __launch_bounds__(kThreads, DIM == 3 && JAC ? 2 : 3) k_tensor(const DiscParams P, const AsmArgs A) {
+    using T = Ten<DIM, SPLIT>;
+    constexpr int NSH = T::NSH, L = T::L, B = T::B, EPW = T::EPW, Pc = DIM, CPL = T::CPL;
     extern __shared__ double smem[];
     const bool tr = P.transient != 0, def = !JAC || A.D != nullptr;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -197,9 +202,9 @@ __global__ void __launch_bounds__(kThreads, 3) k_tensor(const DiscParams P, cons
     double* sv = so + DIM * NSH * EPW;                                          // [NSH][EPW] SCV volumes (general elements)
     auto sE = [&](const int c, const int d) -> double& { return sv[(c * DIM + d) * EPW]; };                    // edge vectors (affine)
     auto sC = [&](const int c, const int d) -> double& { return sv[(DIM * DIM + c * DIM + d) * EPW]; };        // cofactors (affine)
-    // ---- gather: this lane's two corners (the ends of its edge along x)
-    const int l0 = 2 * l;                      // bits (x, y, z) of the first
-    const int c0 = T::corner(l0), c1 = T::corner(l0 + 1);
+    // ---- gather: this lane's corners (the ends of its edge along x; one corner with SPLIT)
+    const int l0 = CPL * l;                    // bits (x, y, z) of the first
+    const int c0 = T::corner(l0), c1 = T::corner(l0 + CPL - 1);
     int32_t nd0 = __ldg(conn + c0), nd1 = __ldg(conn + c1);
 #ifdef NSFV1_BOUNDS_CHECK
     {
@@ -212,16 +217,16 @@ __global__ void __launch_bounds__(kThreads, 3) k_tensor(const DiscParams P, cons
 #pragma unroll
     for (int d = 0; d < DIM; ++d) {
         sx[(d * NSH + l0) * EPW] = __ldg(A.coords + (int64_t)nd0 * DIM + d);
-        sx[(d * NSH + l0 + 1) * EPW] = __ldg(A.coords + (int64_t)nd1 * DIM + d);
+        if (CPL == 2) sx[(d * NSH + l0 + 1) * EPW] = __ldg(A.coords + (int64_t)nd1 * DIM + d);
         if (tr && def) {
             so[(d * NSH + l0) * EPW] = __ldg(A.Uold + (int64_t)nd0 * B + d);
-            so[(d * NSH + l0 + 1) * EPW] = __ldg(A.Uold + (int64_t)nd1 * B + d);
+            if (CPL == 2) so[(d * NSH + l0 + 1) * EPW] = __ldg(A.Uold + (int64_t)nd1 * B + d);
         }
     }
 #pragma unroll
     for (int f = 0; f < B; ++f) {
         su[(f * NSH + l0) * EPW] = __ldg(A.U + (int64_t)nd0 * B + f);
-        su[(f * NSH + l0 + 1) * EPW] = __ldg(A.U + (int64_t)nd1 * B + f);
+        if (CPL == 2) su[(f * NSH + l0 + 1) * EPW] = __ldg(A.U + (int64_t)nd1 * B + f);
     }
     __syncwarp();
     const double nu = A.nuElem ? __ldg(A.nuElem + e) : P.nu;
@@ -231,7 +236,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_tensor(const DiscParams P, cons
     if (tr) idt = 1.0 / P.dt;
     const double js = tr ? P.dt : 1.0;
     const int upw = P.convUpwind;
-    const int pb = l & 1, pc = l >> 1;
+    const int pb = l & 1, pc = DIM == 3 ? l >> 1 : 0, ax = SPLIT ? l >> 1 : 0;
     bool ok = true;
     double* sblk = smem + (size_t)warp * T::warp_doubles(JAC) + T::DOUBLES * EPW;   // [32][STRIDE] (JAC)
 
@@ -276,7 +281,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_tensor(const DiscParams P, cons
             }
         } else {
 #pragma unroll 1
-            for (int k = 0; k < 2; ++k) {
+            for (int k = 0; k < CPL; ++k) {
                 // corner - edge midpoint - centre - edge midpoint: half the cross product of the
                 // diagonals (centre - corner) and (midpoint - midpoint)
                 double x0[2], x1[2], x2[2], x3[2];
@@ -296,7 +301,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_tensor(const DiscParams P, cons
 
     // ---- one SCVF per axis a; b, c the next axes in cyclic order
 #pragma unroll 1
-    for (int a = 0; a < DIM; ++a) {
+    for (int a = ax; a < (SPLIT ? ax + 1 : DIM); ++a) {
         const int sa = 1 << a, sb = 1 << (DIM == 3 ? (a + 1) % 3 : 1 - a), sc = DIM == 3 ? 1 << ((a + 2) % 3) : 0;
         // bits of corner r of the edge frame
         const int near = (pb ? sb : 0) + (pc ? sc : 0);
@@ -564,13 +569,22 @@ __global__ void __launch_bounds__(kThreads, 3) k_tensor(const DiscParams P, cons
             }
             double* __restrict__ dl = A.D + (int64_t)__ldg(conn + clow) * B;
             double* __restrict__ dh = A.D + (int64_t)__ldg(conn + chigh) * B;
-            if (valid)
+            auto reduce = [&]() {
 #pragma unroll
-            for (int f = 0; f < B; ++f) {
-                double v = f < DIM ? flux[f < DIM ? f : 0] : contN * rho;
-                if (tr) v *= js;
-                atomicAdd(dl + f, v);
-                atomicAdd(dh + f, flip_sign(v));
+                for (int f = 0; f < B; ++f) {
+                    double v = f < DIM ? flux[f < DIM ? f : 0] : contN * rho;
+                    if (tr) v *= js;
+                    atomicAdd(dl + f, v);
+                    atomicAdd(dh + f, flip_sign(v));
+                }
+            };
+            if constexpr (SPLIT) {
+                if (valid && ax == 0) reduce();
+                __syncwarp();
+                if (valid && ax == 1) reduce();
+                __syncwarp();
+            } else {
+                if (valid) reduce();
             }
         }
         if constexpr (JAC) {
@@ -623,15 +637,20 @@ __global__ void __launch_bounds__(kThreads, 3) k_tensor(const DiscParams P, cons
 #pragma unroll
                     for (int i = 0; i < T::BB; ++i) sblk[lane * T::STRIDE + i] = Bk[i / B][i % B];
                     __syncwarp();
+                    auto reduce = [&](const int turn) {
 #pragma unroll
-                    for (int j = 0; j < T::BB; ++j) {
-                        const int idx = j * 32 + lane, blk = idx / T::BB, ent = idx - blk * T::BB;
-                        const double v = sblk[blk * T::STRIDE + ent];
-                        const int32_t a0 = __shfl_sync(0xffffffffu, ql[r], blk), a1 = __shfl_sync(0xffffffffu, qh[r], blk);
-                        if (a0 >= 0) atomicAdd(vals + (int64_t)a0 * T::BB + ent, v);
-                        if (a1 >= 0) atomicAdd(vals + (int64_t)a1 * T::BB + ent, flip_sign(v));
-                    }
-                    __syncwarp();
+                        for (int j = 0; j < T::BB; ++j) {
+                            const int idx = j * 32 + lane, blk = idx / T::BB, ent = idx - blk * T::BB;
+                            const double v = sblk[blk * T::STRIDE + ent];
+                            const int32_t a0 = __shfl_sync(0xffffffffu, ql[r], blk), a1 = __shfl_sync(0xffffffffu, qh[r], blk);
+                            if (SPLIT && ((blk >> 1) & 1) != turn) continue;
+                            if (a0 >= 0) atomicAdd(vals + (int64_t)a0 * T::BB + ent, v);
+                            if (a1 >= 0) atomicAdd(vals + (int64_t)a1 * T::BB + ent, flip_sign(v));
+                        }
+                        __syncwarp();
+                    };
+                    reduce(0);
+                    if constexpr (SPLIT) reduce(1);
                 }
             }
         }
@@ -640,10 +659,10 @@ __global__ void __launch_bounds__(kThreads, 3) k_tensor(const DiscParams P, cons
     }
     if (!valid) return;
     if (!ok) atomicOr(A.err, 1);
-    // ---- mass (implicit Euler) and source parts of this lane's two corners
+    // ---- mass (implicit Euler) and source parts of this lane's corners
     if (tr || (def && P.hasSource)) {
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {
+        for (int k = 0; k < CPL; ++k) {
             const double vr = (AFFINE ? vol : sv[(l0 + k) * EPW]) * rho;
             const int c = k ? c1 : c0;
             if (def) {

@@ -86,6 +86,27 @@ def test_matches_oracle(cuda, kind, stab, upwind):
             assert torch.equal(D, D3) and torch.equal(J, J2), "not the same bits"
 
 
+@pytest.mark.parametrize("n", [68, 142])
+def test_quads_around_the_lane_split(cuda, n):
+    """Colours just below and above the element count at which a lane takes both directions again."""
+    import torch
+
+    t, x, c = make("quad-m", n)
+    discs = (NavierStokesFV1(dim=2), oracle.Oracle(2))
+    for d in discs:
+        d.set_kinematic_viscosity(0.02)
+        d.set_upwind("full")
+        d.set_stabilization("flow")
+        d.set_mesh(t, x, c)
+    U = 2 * mesh.uniform(3, x.shape[0] * 3) - 1
+    Dref, Jref = discs[1].assemble(U.reshape(-1, 3))
+    u = torch.from_numpy(U).to(cuda)
+    D, J = torch.empty_like(u), torch.empty(Jref.size, dtype=torch.float64, device=cuda)
+    discs[0].assemble_defect_jacobian(u, D, J)
+    assert rel_err(D.cpu().numpy().reshape(Dref.shape), Dref) <= TOL64
+    assert rel_err(J.cpu().numpy().reshape(Jref.shape), Jref) <= TOL64
+
+
 @pytest.mark.parametrize("kind,n", [("quad", 6), ("hex-j", 3), ("tri", 6)])
 def test_elem_viscosity_and_zero_state(cuda, kind, n):
     """Per-element viscosity, and the state at rest (every upwind ties)."""

@@ -443,7 +443,7 @@ def main():
         ach_wi = prof["fp64_inst_per_element"] * n_el / 32.0 / (ms64 * 1e-3)
         fp64_pipe = {"achieved_warp_inst_per_s": ach_wi, "peak_warp_inst_per_s": peak_wi, "frac": ach_wi / peak_wi,
                      "fp64_inst_per_element": prof["fp64_inst_per_element"], "sm_mhz": sm_mhz,
-                     "source": "FP64 instruction count per element from ncu (profiles/k_defect_jacobian_hex_fp64.md)"}
+                     "source": "FP64 instruction count per element from ncu (profiles/k_tensor_hex_fp64.md)"}
     traffic32 = prof.get("jacobian_f32_bytes_per_assembly")
     # the colour launches of one assembly (the rooflines' figures are per launch)
     n_launch = int(d.pattern_info().get("n_colors", prof.get("launches_per_assembly", 8)))

@@ -1295,8 +1295,10 @@ static int gmres(Disc& D, const MT* J, const MT* Dinv, const double* rhs, double
     unsigned* counters = reinterpret_cast<unsigned*>(W.scal + 200);
     const int g = grid_for(n), gRows = grid_for(D.nNodes, kGmT);
     const int gRed = (int)std::min<int64_t>(kGmBlocks, (n + kGmT - 1) / kGmT);
-    const size_t smemMax = (size_t)(m + 1) * kGmT * sizeof(double);
-    if (!D.cuda_ok(cudaFuncSetAttribute(k_gm_axpy_dots, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemMax), "gmres setup")) return -1;
+    // the attribute belongs to the kernel, not to this solve: every solve sets the same value, so a
+    // solve with another restart length on another thread cannot take it away
+    constexpr int smemMax = (kGmMaxM + 1) * kGmT * (int)sizeof(double);
+    if (!D.cuda_ok(cudaFuncSetAttribute(k_gm_axpy_dots, cudaFuncAttributeMaxDynamicSharedMemorySize, smemMax), "gmres setup")) return -1;
     k_fill<double><<<g, 256, 0, s>>>(n, x, 0.0);
     cudaMemsetAsync(G, 0, sizeof(double) * G_H1, s);
     cudaMemsetAsync(counters, 0, 4 * sizeof(unsigned), s);
@@ -1305,7 +1307,7 @@ static int gmres(Disc& D, const MT* J, const MT* Dinv, const double* rhs, double
     bool first = true;
     while (it < maxit) {
         // V_0 = rhs - J x (x = 0 in the first cycle)
-        if (!first) spmv<MT, double>(D, J, x, w, s);
+        if (!first && !D.cuda_ok(spmv<MT, double>(D, J, x, w, s), "gmres launch")) return -1;
         k_gm_start<<<gRed, kGmT, 0, s>>>(n, rhs, first ? nullptr : w, Vb, W.red, counters, G, rtol);
         first = false;
         int j = 0, done = 0;
@@ -1319,7 +1321,8 @@ static int gmres(Disc& D, const MT* J, const MT* Dinv, const double* rhs, double
                 const int jEnd = q > 0 ? j : 0;
                 if (D.dim == 3) k_gm_prec<MT, 4><<<gRows + 1, kGmT, 0, s>>>(D.nNodes, G, Vj, Dinv, Zj, jEnd, m, rtol);
                 else k_gm_prec<MT, 3><<<gRows + 1, kGmT, 0, s>>>(D.nNodes, G, Vj, Dinv, Zj, jEnd, m, rtol);
-                spmv<MT, double>(D, J, Zj, wj, s, G + G_DONE);
+                // the product's status is also that of the launches before it
+                if (!D.cuda_ok(spmv<MT, double>(D, J, Zj, wj, s, G + G_DONE), "gmres launch")) return -1;
                 k_gm_dots<<<gRed, kGmT, 0, s>>>(n, j, Vb, wj, W.red, counters, G);
                 k_gm_axpy_dots<<<gRed, kGmT, (size_t)(j + 2) * kGmT * sizeof(double), s>>>(n, j, Vb, wj, W.red, counters, G);
                 k_gm_end<<<gRed, kGmT, 0, s>>>(n, j, Vb, wj, W.red, counters, G);

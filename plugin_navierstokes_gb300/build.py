@@ -31,7 +31,8 @@ def nvcc_path() -> str:
 
 
 def _flags(extra: list[str] | None = None) -> list[str]:
-    f = ARCH + ["-O3", "-lineinfo", "-std=c++17", "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC",
+    # 2809: the value of a [[nodiscard]] function (a launch status) is dropped
+    f = ARCH + ["-O3", "-lineinfo", "-std=c++17", "--expt-relaxed-constexpr", "-diag-error", "2809", "-Xcompiler", "-fPIC",
                 "-Xcompiler", "-ffp-contract=on", "-I", str(HERE.parent / "include")]
     return f + (extra or [])
 

@@ -1072,8 +1072,9 @@ static inline int grid_for(int64_t n, int t = 256) { return (int)((n + t - 1) / 
 // to 88.2 us (8 -> 4 lanes; 2 lanes: 87.9 us, 1 lane: 105.0 us, loads uncoalesced).
 template <int b> constexpr int spmv_lanes() { return b == 4 ? 8 : 4; }
 
+// (the status is that of every launch since the last one that was read: not to be dropped)
 template <typename MT, typename VT>
-static cudaError_t spmv(const Disc& D, const MT* vals, const VT* x, VT* y, cudaStream_t s, const double* gate = nullptr) {
+[[nodiscard]] static cudaError_t spmv(const Disc& D, const MT* vals, const VT* x, VT* y, cudaStream_t s, const double* gate = nullptr) {
     const int64_t nR = D.nNodes;
     const int b = D.dim + 1;
     if constexpr (std::is_same<MT, double>::value) {
@@ -1095,7 +1096,7 @@ static cudaError_t spmv(const Disc& D, const MT* vals, const VT* x, VT* y, cudaS
 }
 
 // y = A x for an FP32 matrix and split x
-static cudaError_t spmv_split(const Disc& D, const float* vals, const float2* xs, double* y, cudaStream_t s, const double* gate = nullptr) {
+[[nodiscard]] static cudaError_t spmv_split(const Disc& D, const float* vals, const float2* xs, double* y, cudaStream_t s, const double* gate = nullptr) {
     const int64_t nR = D.nNodes;
     constexpr int G4 = spmv_lanes<4>(), G3 = spmv_lanes<3>();
     if (D.dim == 3) k_bsr_mv_split<4, G4><<<grid_for(nR * G4), 256, 0, s>>>(nR, D.d_rowPtr, D.d_colIdx, vals, xs, y, gate);
@@ -1172,7 +1173,7 @@ static constexpr int kBicgBatch = 16;
 static unsigned* bicg_counters(Workspace& W) { return reinterpret_cast<unsigned*>(W.scal + 200); }
 
 template <typename MT, int b>
-static void bicg_iteration(Disc& D, const MT* J, const MT* Dinv, double* const (&V)[10], double* x, double nr0, double rtol, cudaStream_t s) {
+[[nodiscard]] static cudaError_t bicg_iteration(Disc& D, const MT* J, const MT* Dinv, double* const (&V)[10], double* x, double nr0, double rtol, cudaStream_t s) {
     Workspace& W = D.ws;
     double *r = V[0], *r0 = V[1], *p = V[2], *v = V[3], *sv = V[4], *t = V[5], *ph = V[6], *shv = V[7];
     float2* phs = reinterpret_cast<float2*>(V[8]);   // split copies of ph and shv (FP32 matrices)
@@ -1182,20 +1183,18 @@ static void bicg_iteration(Disc& D, const MT* J, const MT* Dinv, double* const (
     const int64_t nR = D.nNodes, n = W.n;
     const int gn = grid_for(nR);
     auto mv = [&](const double* xd, const float2* xsplit, double* y) {
-        if constexpr (std::is_same<MT, float>::value) {
-            spmv_split(D, J, xsplit, y, s, done);
-        } else {
-            spmv<MT, double>(D, J, xd, y, s, done);
-        }
+        if constexpr (std::is_same<MT, float>::value) return spmv_split(D, J, xsplit, y, s, done);
+        else return spmv<MT, double>(D, J, xd, y, s, done);
     };
     unsigned* counters = bicg_counters(W);
     k_bicg_p_prec<MT, b><<<gn, 256, 0, s>>>(nR, S, r, v, p, Dinv, ph, phs);
-    mv(ph, phs, v);
+    if (const cudaError_t e = mv(ph, phs, v); e != cudaSuccess) return e;
     k_bicg_dot_alpha<<<kRedBlocks, kRedThreads, 0, s>>>(n, r0, v, W.red, counters + 0, S);
     k_bicg_s_prec<MT, b><<<gn, 256, 0, s>>>(nR, S, r, v, sv, Dinv, shv, shs);
-    mv(shv, shs, t);
+    if (const cudaError_t e = mv(shv, shs, t); e != cudaSuccess) return e;
     k_bicg_dot_omega<<<kRedBlocks, kRedThreads, 0, s>>>(n, t, sv, W.red, counters + 1, S);
     k_bicg_x_end<<<kRedBlocks, kRedThreads, 0, s>>>(n, S, ph, shv, sv, t, r0, x, r, W.red, counters + 2, nr0, rtol);
+    return cudaGetLastError();
 }
 
 // The Krylov vectors are FP64 whatever the precision MT of the stored Jacobian:
@@ -1246,11 +1245,10 @@ static int bicgstab(Disc& D, const MT* J, const MT* Dinv, const double* rhs, dou
                 dots<VT, 1>(n, a, c, W.red, s);
                 k_bicg_beta<<<1, kRedThreads, 0, s>>>(W.red, kRedBlocks, S);
             }
-            if (b == 4) bicg_iteration<MT, 4>(D, J, Dinv, V, x, nr0, rtol, s);
-            else bicg_iteration<MT, 3>(D, J, Dinv, V, x, nr0, rtol, s);
+            const cudaError_t e = b == 4 ? bicg_iteration<MT, 4>(D, J, Dinv, V, x, nr0, rtol, s) : bicg_iteration<MT, 3>(D, J, Dinv, V, x, nr0, rtol, s);
+            if (!D.cuda_ok(e, "bicgstab launch")) return -1;
         }
         needBeta = false;
-        if (!D.cuda_ok(cudaGetLastError(), "bicgstab launch")) return -1;
         if (!read_scal(D, 0, S_NSCAL, s)) return -1;
         it = (int)W.hscal[S_ITER];
         const double nr = std::sqrt(W.hscal[S_NR2]);

@@ -6,6 +6,7 @@
 // reductions accumulate in FP64 with a fixed grid and a fixed summation tree,
 // so results are bitwise reproducible run to run.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <type_traits>
@@ -682,7 +683,7 @@ __global__ void k_set_dirichlet(int64_t n, const int32_t* __restrict__ rows, con
 }
 
 // GMRES -----------------------------------------------------------------------
-// One iteration is five launches and no host read: the scalar work (Gram-Schmidt
+// One iteration is five launches and no wait for the host: the scalar work (Gram-Schmidt
 // sums, Givens rotations, stop tests) is done by the last block of each reduction.
 // Four FP64 multiply-adds per basis entry on a pipe that takes a warp instruction
 // every 19 clocks per SM (about 14 us an iteration at 192^2 quadrilaterals, n =
@@ -818,7 +819,8 @@ __device__ __forceinline__ void gm_range(const int64_t n, int64_t& i0, int64_t& 
 // start of a cycle: V_0 = rhs - J x (w = J x, or null for x = 0) and its norm; the last block
 // sets the stop state (converged at the start of a cycle, zero right-hand side) and 1 / beta
 __global__ void __launch_bounds__(kGmT) k_gm_start(int64_t n, const double* __restrict__ rhs, const double* __restrict__ w, double* __restrict__ V0,
-                                                   double* __restrict__ partials, unsigned* counter, double* G, double rtol) {
+                                                   double* __restrict__ partials, unsigned* counter, double* G, volatile double* host,
+                                                   double rtol) {
     double acc = 0.0;
     int64_t i0, i1;
     gm_range(n, i0, i1);
@@ -836,8 +838,16 @@ __global__ void __launch_bounds__(kGmT) k_gm_start(int64_t n, const double* __re
     G[G_J] = 0.0;
     G[G_INV] = 1.0 / beta;
     G[G_GAM] = beta;
-    // beta = 0, or below the tolerance: nothing to iterate (the host leaves the loop)
-    G[G_DONE] = (beta0 == 0.0 || G[G_RELRES] < rtol) ? GM_CYCLE_END : 0.0;
+    // a zero right-hand side, or below the tolerance: nothing to iterate (the host leaves the loop).
+    // With rtol = 0 a restart at beta = 0 goes on and ends as a breakdown.
+    const bool done = beta0 == 0.0 || G[G_RELRES] < rtol;
+    G[G_DONE] = done ? GM_CYCLE_END : 0.0;
+    host[G_RELRES] = G[G_RELRES];
+    host[G_J] = 0.0;
+    if (done) {
+        __threadfence_system();
+        host[G_DONE] = GM_CYCLE_END;
+    }
 }
 
 // h1[k] = (V_k, w), k <= j: a tile of w goes to shared memory, each warp streams the tiles of
@@ -965,7 +975,8 @@ __global__ void __launch_bounds__(kGmT) k_gm_end(int64_t n, int j, const double*
 // the scalar end of iteration j (one block): the Hessenberg column h1 + h2, the Givens
 // rotations, the residual estimate and the stop tests. The rotations are one serial chain of
 // FP64 operations (64 clocks each): its inputs come to shared memory first.
-__device__ __forceinline__ void gm_givens(double* G, const int j, const int m, const double rtol) {
+// The host follows in pinned memory: the iteration count, and at a stop the state, then G_DONE.
+__device__ __forceinline__ void gm_givens(double* G, volatile double* host, const int j, const int m, const double rtol) {
     __shared__ double hc[kGmMaxM + 1], cs[kGmMaxM], sn[kGmMaxM];
     const int t = threadIdx.x;
     if (t <= j) hc[t] = G[G_H1 + t] + G[G_H2 + t];
@@ -989,37 +1000,45 @@ __device__ __forceinline__ void gm_givens(double* G, const int j, const int m, c
         const double relres = fabs(sj * gj) / beta0;
         G[G_RELRES] = relres;
         G[G_IT] = it + 1.0;
-        if (!isfinite(relres)) G[G_DONE] = GM_NONFINITE;
-        else if (relres < rtol || hn == 0.0) G[G_DONE] = GM_CYCLE_END;
+        const int done = !isfinite(relres) ? GM_NONFINITE : relres < rtol || hn == 0.0 ? GM_CYCLE_END : 0;
+        host[G_RELRES] = relres;
+        host[G_J] = j + 1;
+        host[G_IT] = it + 1.0;
+        if (done) {
+            G[G_DONE] = done;
+            __threadfence_system();
+            host[G_DONE] = done;
+        }
     }
     __syncthreads();
     if (t <= j) G[G_HES + t * m + j] = hc[t];   // H[k * m + column]
 }
 
-__global__ void __launch_bounds__(kGmT) k_gm_givens(double* G, int j, int m, double rtol) {
-    if (G[G_DONE] == 0.0) gm_givens(G, j, m, rtol);
+__global__ void __launch_bounds__(kGmT) k_gm_givens(double* G, double* host, int j, int m, double rtol) {
+    if (G[G_DONE] == 0.0) gm_givens(G, host, j, m, rtol);
 }
 
 // V_j *= 1 / norm; Z_j = Dinv V_j (the point-block Jacobi apply of k_prec, same summation).
 // The last block ends iteration j - 1 (gm_givens) meanwhile: up to 5 us of serial FP64 that
-// would otherwise stand at the tail of k_gm_end. A stop found there lets this kernel's writes
-// stand (V_j and Z_j are not used after a stop).
+// would otherwise stand at the tail of k_gm_end. V_j and Z_j are not used after a stop: the other
+// blocks leave them where they see one (the stop that this launch finds may or may not reach them).
 template <typename MT, int b>
-__global__ void __launch_bounds__(kGmT) k_gm_prec(int64_t nRows, double* G, double* __restrict__ Vj, const MT* __restrict__ Dinv,
-                                                  double* __restrict__ Zj, int j, int m, double rtol) {
+__global__ void __launch_bounds__(kGmT) k_gm_prec(int64_t nRows, double* G, double* host, double* __restrict__ Vj,
+                                                  const MT* __restrict__ Dinv, double* __restrict__ Zj, int j, int m, double rtol) {
     if (blockIdx.x == gridDim.x - 1) {
-        if (j > 0 && G[G_DONE] == 0.0) gm_givens(G, j - 1, m, rtol);
+        if (j > 0 && G[G_DONE] == 0.0) gm_givens(G, host, j - 1, m, rtol);
         return;
     }
     const int64_t r = (int64_t)blockIdx.x * kGmT + threadIdx.x;
     if (r >= nRows) return;
-    const double inv = G[G_INV];
+    // (the test after the loads: one round trip to L2 instead of two)
+    const double inv = G[G_INV], done = __ldcg(G + G_DONE);
     double x[b];
 #pragma unroll
-    for (int i = 0; i < b; ++i) {
-        x[i] = Vj[r * b + i] * inv;
-        Vj[r * b + i] = x[i];
-    }
+    for (int i = 0; i < b; ++i) x[i] = Vj[r * b + i] * inv;
+    if (done != 0.0) return;
+#pragma unroll
+    for (int i = 0; i < b; ++i) Vj[r * b + i] = x[i];
     const MT* M = Dinv + r * b * b;
 #pragma unroll
     for (int i = 0; i < b; ++i) {
@@ -1275,9 +1294,24 @@ static int bicgstab(Disc& D, const MT* J, const MT* Dinv, const double* rhs, dou
     return maxit;
 }
 
-// Iterations queued between two host reads of the solver state (as kBicgBatch): the kernels of
-// a later queued iteration return at once after a stop.
-static constexpr int kGmresBatch = 16;
+// Iterations that the host queues ahead of the one that has ended last (G_IT in pinned memory). The
+// kernels queued behind a stop return at once, about 12 us an iteration: with 16 iterations
+// queued between two copies of the state, a solve that stops after one iteration took twice
+// the time of three host reads per iteration (10^3 hexahedra: 442 and 215 us; now 190). A
+// copy of the state in the stream costs 7 us, pinned memory that the device writes nothing measurable
+// (192^2 quadrilaterals, 45 iterations: 3.02 ms with three copies, 3.00 ms now).
+static constexpr int kGmresAhead = 3;
+
+// waits until the device has ended 'iters' iterations, has stopped, or has nothing queued any more
+static bool gmres_wait(Disc& D, const volatile double* host, int iters, cudaStream_t s) {
+    for (int spin = 1; host[G_IT] < iters && host[G_DONE] == 0.0; ++spin) {
+        if (spin % 256) continue;
+        const cudaError_t e = cudaStreamQuery(s);
+        if (e == cudaSuccess) break;
+        if (e != cudaErrorNotReady) return D.cuda_ok(e, "gmres state");
+    }
+    return true;
+}
 
 // restarted GMRES(m), right preconditioned, classical Gram-Schmidt with one
 // re-orthogonalisation pass; Hessenberg least squares (Givens) on the device.
@@ -1300,42 +1334,42 @@ static int gmres(Disc& D, const MT* J, const MT* Dinv, const double* rhs, double
     k_fill<double><<<g, 256, 0, s>>>(n, x, 0.0);
     cudaMemsetAsync(G, 0, sizeof(double) * G_H1, s);
     cudaMemsetAsync(counters, 0, 4 * sizeof(unsigned), s);
-    *relres = 1.0;
+    double* host = W.hscal + 128;   // pinned: the device writes the state here
+    volatile double* state = host;
+    state[G_DONE] = state[G_J] = state[G_IT] = 0.0;
+    *relres = state[G_RELRES] = 1.0;
     int it = 0;
     bool first = true;
     while (it < maxit) {
         // V_0 = rhs - J x (x = 0 in the first cycle)
         if (!first && !D.cuda_ok(spmv<MT, double>(D, J, x, w, s), "gmres launch")) return -1;
-        k_gm_start<<<gRed, kGmT, 0, s>>>(n, rhs, first ? nullptr : w, Vb, W.red, counters, G, rtol);
+        k_gm_start<<<gRed, kGmT, 0, s>>>(n, rhs, first ? nullptr : w, Vb, W.red, counters, G, host, rtol);
         first = false;
-        int j = 0, done = 0;
-        while (!done && j < m && it < maxit) {
-            const int K = std::min(std::min(kGmresBatch, m - j), maxit - it);
-            for (int q = 0; q < K; ++q, ++j) {
-                double* Vj = Vb + (int64_t)j * n;
-                double* Zj = Zb + (int64_t)j * n;
-                double* wj = Vj + n;
-                // the first of a batch finds iteration j - 1 ended already
-                const int jEnd = q > 0 ? j : 0;
-                if (D.dim == 3) k_gm_prec<MT, 4><<<gRows + 1, kGmT, 0, s>>>(D.nNodes, G, Vj, Dinv, Zj, jEnd, m, rtol);
-                else k_gm_prec<MT, 3><<<gRows + 1, kGmT, 0, s>>>(D.nNodes, G, Vj, Dinv, Zj, jEnd, m, rtol);
-                // the product's status is also that of the launches before it
-                if (!D.cuda_ok(spmv<MT, double>(D, J, Zj, wj, s, G + G_DONE), "gmres launch")) return -1;
-                k_gm_dots<<<gRed, kGmT, 0, s>>>(n, j, Vb, wj, W.red, counters, G);
-                k_gm_axpy_dots<<<gRed, kGmT, (size_t)(j + 2) * kGmT * sizeof(double), s>>>(n, j, Vb, wj, W.red, counters, G);
-                k_gm_end<<<gRed, kGmT, 0, s>>>(n, j, Vb, wj, W.red, counters, G);
-            }
-            k_gm_givens<<<1, kGmT, 0, s>>>(G, j - 1, m, rtol);
-            if (!D.cuda_ok(cudaGetLastError(), "gmres launch")) return -1;
-            if (!D.cuda_ok(cudaMemcpyAsync(W.hscal, G, sizeof(double) * G_H1, cudaMemcpyDeviceToHost, s), "gmres state") ||
-                !D.cuda_ok(cudaStreamSynchronize(s), "gmres state"))
-                return -1;
-            done = (int)W.hscal[G_DONE];
-            it = (int)W.hscal[G_IT];
-            *relres = W.hscal[G_RELRES];
+        int j = 0;
+        for (; j < m && it + j < maxit && state[G_DONE] == 0.0; ++j) {
+            double* Vj = Vb + (int64_t)j * n;
+            double* Zj = Zb + (int64_t)j * n;
+            double* wj = Vj + n;
+            // ends iteration j - 1 too
+            if (D.dim == 3) k_gm_prec<MT, 4><<<gRows + 1, kGmT, 0, s>>>(D.nNodes, G, host, Vj, Dinv, Zj, j, m, rtol);
+            else k_gm_prec<MT, 3><<<gRows + 1, kGmT, 0, s>>>(D.nNodes, G, host, Vj, Dinv, Zj, j, m, rtol);
+            // the product's status is also that of the launches before it
+            if (!D.cuda_ok(spmv<MT, double>(D, J, Zj, wj, s, G + G_DONE), "gmres launch")) return -1;
+            k_gm_dots<<<gRed, kGmT, 0, s>>>(n, j, Vb, wj, W.red, counters, G);
+            k_gm_axpy_dots<<<gRed, kGmT, (size_t)(j + 2) * kGmT * sizeof(double), s>>>(n, j, Vb, wj, W.red, counters, G);
+            k_gm_end<<<gRed, kGmT, 0, s>>>(n, j, Vb, wj, W.red, counters, G);
+            if (!gmres_wait(D, state, it + j + 1 - kGmresAhead, s)) return -1;
         }
+        if (state[G_DONE] == 0.0) {
+            k_gm_givens<<<1, kGmT, 0, s>>>(G, host, j - 1, m, rtol);
+            if (!D.cuda_ok(cudaGetLastError(), "gmres launch") || !D.cuda_ok(cudaStreamSynchronize(s), "gmres state")) return -1;
+        }
+        std::atomic_thread_fence(std::memory_order_acquire);   // the state was written before G_DONE
+        const int done = (int)state[G_DONE], jn = (int)state[G_J];
+        it = (int)state[G_IT];
+        *relres = state[G_RELRES];
+        state[G_DONE] = 0.0;   // for the next cycle
         if (done == GM_NONFINITE) return -1;
-        const int jn = (int)W.hscal[G_J];
         if (jn == 0) return it;   // zero right-hand side, or converged at the start of the cycle
         // y = H^-1 gam ; x += Z y
         k_gm_y<<<1, 32, 0, s>>>(G, m);

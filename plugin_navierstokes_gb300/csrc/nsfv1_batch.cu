@@ -785,7 +785,7 @@ int batched_newton(Disc& D, double* u, const double* u_old, double dt, const nsf
     if (W.prec != prec || W.n != n || W.m != m || W.nInst != nInst || W.nnzb != nnzb) {
         W.release();
         const size_t vt = sizeof(VT);
-        auto al = [&](auto*& ptr, size_t bytes) { return D.cuda_ok(cudaMalloc((void**)&ptr, bytes), "batch workspace"); };
+        auto al = [&](auto*& ptr, size_t bytes) { return D.cuda_ok(D.device_malloc((void**)&ptr, bytes), "batch workspace"); };
         if (!al(W.D, n * 8) || !al(W.Dt, n * 8) || !al(W.Ut, n * 8) || !al(W.nrm, nInst * 8) || !al(W.lambda, nInst * 8) ||
             !al(W.relres, nInst * 8) || !al(W.J, D.colIdx.size() * b * b * vt) || !al(W.Dinv, (size_t)D.nNodes * b * b * vt) ||
             !al(W.V, (size_t)(m + 1) * n * vt) || !al(W.t, n * vt) || !al(W.x, n * vt) || !al(W.q, n * vt) || !al(W.s, n * vt) ||
@@ -822,8 +822,9 @@ int batched_newton(Disc& D, double* u, const double* u_old, double dt, const nsf
     if (useMG) {
         for (size_t l = 1; l < BS->levels.size(); ++l) {
             Level& L = BS->levels[l];
-            if (L.prec == prec) continue;
             Disc& C = *L.disc;
+            if (prec == NSFV1_F32) C.ensure_diag_stage(s);
+            if (L.prec == prec) continue;
             const int64_t nc = C.nNodes;
             auto f = [](auto*& q) { if (q) cudaFree((void*)q); q = nullptr; };
             f(L.J); f(L.Dinv); f(L.x); f(L.r); f(L.s); f(L.x2);

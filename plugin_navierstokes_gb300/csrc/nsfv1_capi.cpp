@@ -85,51 +85,70 @@ void Disc::free_mesh() {
     outflowHost.clear();
     bndFluxHost.clear();
     dfree(d_instNode0); dfree(d_elemInst); dfree(d_nodeInst); dfree(d_instActive);
+    free_diag_stage();
     dfree(d_diagPtr);
-    d_diagSlot = nullptr; d_diagStage = nullptr;
+    diagTried = false;
     nInst = 0; instNode0.clear(); instSkip = false;
     // the batched solver's levels, graphs and buffers belong to this mesh
     if (batch) { batch_free(batch); batch = nullptr; }
 }
 
+void Disc::free_diag_stage() {
+    dfree(d_diagSlot);
+    d_diagStage = nullptr;
+}
+
 // Staging of the one-launch FP32 Jacobian of a 2D mesh: slot of every (element, corner), a node's
-// slots in the colour order of its elements. Not an error where it cannot be had (an edge in
-// three elements, no memory for the stage): the mesh is then assembled colour by colour.
-bool Disc::setup_diag_stage(const std::vector<int32_t>& nodeElemPtr) {
-    dfree(d_diagPtr);
-    d_diagSlot = nullptr; d_diagStage = nullptr;
-    if (dim != 2) return true;
-    // on the device, where the mesh is already (host loops took a sixth of set_mesh); one allocation:
-    // offsets, slots, stage, and the stage holds the counters meanwhile
-    const size_t nPtr = ((size_t)nNodes + 1 + 3) / 4 * 4, nSlot = ((size_t)nElems * nsh + 3) / 4 * 4;
+// slots in the colour order of its elements. Made at the first FP32 Jacobian (before any capture):
+// it holds nearly as much as the FP32 matrix, and a handle that only assembles FP64 never needs it.
+// Not an error where it cannot be had (an edge in three elements, no memory for the stage): the
+// mesh is then assembled colour by colour.
+void Disc::ensure_diag_stage(cudaStream_t s) {
+    if (diagTried || dim != 2) return;
+    diagTried = true;
+    // on the device, where the mesh is already; one allocation: slots, then the stage, which holds the
+    // counters meanwhile
+    const size_t nSlot = ((size_t)nElems * nsh + 3) / 4 * 4;
     const size_t nStage = std::max((size_t)nElems * nsh * 9, std::max(colIdx.size(), (size_t)nNodes) + 1);
     int32_t* buf = nullptr;
-    if (cudaMalloc((void**)&buf, (nPtr + nSlot + nStage) * sizeof(int32_t)) != cudaSuccess) { cudaGetLastError(); return true; }
-    int32_t *ptr = buf, *slot = buf + nPtr, *tmp = slot + nSlot;
+    if (cudaMalloc((void**)&buf, (nSlot + nStage) * sizeof(int32_t)) != cudaSuccess) { cudaGetLastError(); return; }
+    int32_t *slot = buf, *tmp = buf + nSlot;
     int many = 1;
-    bool ok = launch_count_blocks(nsh, nElems, d_elemBlk, (int64_t)colIdx.size(), tmp, nullptr) == cudaSuccess &&
-              cudaMemcpy(&many, tmp + colIdx.size(), sizeof(int), cudaMemcpyDeviceToHost) == cudaSuccess;
+    bool ok = launch_count_blocks(nsh, nElems, d_elemBlk, (int64_t)colIdx.size(), tmp, s) == cudaSuccess &&
+              cudaMemcpyAsync(&many, tmp + colIdx.size(), sizeof(int), cudaMemcpyDeviceToHost, s) == cudaSuccess &&
+              cudaStreamSynchronize(s) == cudaSuccess;
     if (ok && !many) {
-        ok = cudaMemcpy(ptr, nodeElemPtr.data(), nodeElemPtr.size() * sizeof(int32_t), cudaMemcpyHostToDevice) == cudaSuccess &&
-             cudaMemset(tmp, 0, (size_t)nNodes * sizeof(int32_t)) == cudaSuccess;
+        ok = cudaMemsetAsync(tmp, 0, (size_t)nNodes * sizeof(int32_t), s) == cudaSuccess;
         for (int c = 0; ok && c < nColors; ++c)
-            ok = launch_assign_slots(nsh, d_colorElems + colorPtr[c], colorPtr[c + 1] - colorPtr[c], d_conn, ptr, tmp, slot, nullptr) == cudaSuccess;
-        if (ok) ok = cudaStreamSynchronize(nullptr) == cudaSuccess;
+            ok = launch_assign_slots(nsh, d_colorElems + colorPtr[c], colorPtr[c + 1] - colorPtr[c], d_conn, d_diagPtr, tmp, slot, s) == cudaSuccess;
     }
     if (ok && !many) {
-        d_diagPtr = ptr; d_diagSlot = slot; d_diagStage = reinterpret_cast<float*>(tmp);
+        d_diagSlot = slot; d_diagStage = reinterpret_cast<float*>(tmp);
     } else {
         cudaGetLastError();
         cudaFree(buf);
     }
-    return true;
+}
+
+// cudaMalloc that gives the staging back where memory is short: what fits without it still does
+cudaError_t Disc::device_malloc(void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && d_diagSlot) {
+        cudaGetLastError();
+        free_diag_stage();
+        e = cudaMalloc(p, bytes);
+    }
+    return e;
 }
 
 // The FP32 Jacobian of all elements in one launch where that is served (it skips no instance);
 // the values are cleared already
 bool Disc::jacobian_f32_at_once(const DiscParams& P, const AsmArgs& whole, cudaStream_t s, bool& served) {
-    served = d_diagStage && !instSkip && !uses_ipshape(P);
-    if (!served) return true;
+    served = false;
+    if (instSkip || uses_ipshape(P)) return true;
+    ensure_diag_stage(s);
+    if (!d_diagStage) return true;
+    served = true;
     AsmArgs a = whole;
     a.elems = nullptr;
     a.count = (int32_t)nElems;
@@ -477,7 +496,7 @@ int nsfv1_set_mesh(nsfv1_disc* h, int elem_type, int64_t n_nodes, const double* 
         D->coordsHost.assign(coords, coords + n_nodes * dim);
         D->connHost.assign(conn, conn + n_elems * nsh);
         D->nuElemHost.clear(); D->dirRowHost.clear(); D->dirValHost.clear(); D->instCells.clear();
-        std::vector<int32_t> nodeElemPtr;
+        std::vector<int32_t> nodeElemPtr;   // offsets of the elements around a node (2D)
         build_pattern(nsh, n_nodes, n_elems, conn, D->rowPtr, D->colIdx, D->elemBlk, dim == 2 ? &nodeElemPtr : nullptr);
         D->nColors = build_coloring(nsh, n_nodes, n_elems, conn, D->color);
         if (D->nColors < 0) { D->fail(NSFV1_ERR_ARGUMENT, "too many element colours"); return D->status; }
@@ -499,7 +518,8 @@ int nsfv1_set_mesh(nsfv1_disc* h, int elem_type, int64_t n_nodes, const double* 
             !D->cuda_ok(dupload(D->d_elemBlk, D->elemBlk.data(), D->elemBlk.size()), "upload elemBlk") ||
             !D->cuda_ok(dupload(D->d_colorElems, D->colorElems.data(), D->colorElems.size()), "upload colours") ||
             !D->cuda_ok(dupload(D->d_rowPtr, D->rowPtr.data(), D->rowPtr.size()), "upload rowPtr") ||
-            !D->cuda_ok(dupload(D->d_colIdx, D->colIdx.data(), D->colIdx.size()), "upload colIdx"))
+            !D->cuda_ok(dupload(D->d_colIdx, D->colIdx.data(), D->colIdx.size()), "upload colIdx") ||
+            !D->cuda_ok(dupload(D->d_diagPtr, nodeElemPtr.data(), nodeElemPtr.size()), "upload node offsets"))
             return D->status;
         {
             std::vector<int32_t> dp(n_nodes);
@@ -515,7 +535,7 @@ int nsfv1_set_mesh(nsfv1_disc* h, int elem_type, int64_t n_nodes, const double* 
             if (!D->cuda_ok(cudaMalloc((void**)&D->d_err, sizeof(int)), "alloc err")) return D->status;
         }
         if (!D->cuda_ok(cudaMemset(D->d_err, 0, sizeof(int)), "memset err")) return D->status;
-        if (!D->ensure_ipws() || !D->setup_diag_stage(nodeElemPtr)) return D->status;
+        if (!D->ensure_ipws()) return D->status;
         D->nDir = 0;
         D->free_workspace();
         D->hasMesh = true;

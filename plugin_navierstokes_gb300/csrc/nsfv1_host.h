@@ -47,10 +47,11 @@ struct Disc {
     double* d_coords = nullptr;
     int32_t *d_conn = nullptr, *d_elemBlk = nullptr, *d_colorElems = nullptr, *d_rowPtr = nullptr, *d_colIdx = nullptr;
     // 2D meshes whose off-diagonal blocks get at most two contributions: the staged diagonal blocks
-    // of the one-launch FP32 Jacobian (nsfv1_jac_lanes.cu), one allocation owned by d_diagPtr; null
-    // where it is not served
-    int32_t *d_diagPtr = nullptr, *d_diagSlot = nullptr;
+    // of the one-launch FP32 Jacobian (nsfv1_jac_lanes.cu), one allocation owned by d_diagSlot, made at
+    // the first FP32 Jacobian; null where it is not served
+    int32_t *d_diagPtr = nullptr, *d_diagSlot = nullptr;   // [nNodes + 1] offsets of a node's slots, slots
     float* d_diagStage = nullptr;
+    bool diagTried = false;
     int32_t* d_diagPos = nullptr;   // block index of each row's diagonal block
     double* d_nuElem = nullptr;     // per-element viscosity (nsfv1_set_elem_viscosity), or null
     // independent instances (nsfv1_set_instances): node ranges, element -> instance
@@ -109,7 +110,9 @@ struct Disc {
     bool assemble_jacobian(const double* u, const double* u_old, double dt, void* vals, int prec, cudaStream_t s, bool sync = true);
     bool assemble_defect_jacobian(const double* u, const double* u_old, double dt, double* d, void* vals, int prec, cudaStream_t s);
     bool ensure_workspace(int prec, int gmresM);
-    bool setup_diag_stage(const std::vector<int32_t>& nodeElemPtr);   // [nNodes + 1] offsets of the elements around a node
+    void ensure_diag_stage(cudaStream_t s);
+    void free_diag_stage();
+    cudaError_t device_malloc(void** p, size_t bytes);
     bool jacobian_f32_at_once(const DiscParams& P, const AsmArgs& whole, cudaStream_t s, bool& served);
     bool set_dirichlet_values(double* u, cudaStream_t s);   // u[dof] = g for every Dirichlet row
 };

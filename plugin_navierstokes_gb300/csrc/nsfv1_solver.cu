@@ -1159,7 +1159,7 @@ bool Disc::ensure_workspace(int prec, int gmresM) {
     if (ws.prec == prec && ws.n == n && ws.nvec >= nvec) return true;
     free_workspace();
     const size_t vt = prec == NSFV1_F64 ? sizeof(double) : sizeof(float);
-    auto al = [&](auto*& p, size_t bytes) { return cuda_ok(cudaMalloc((void**)&p, bytes), "workspace alloc"); };
+    auto al = [&](auto*& p, size_t bytes) { return cuda_ok(device_malloc((void**)&p, bytes), "workspace alloc"); };
     if (!al(ws.D, n * 8) || !al(ws.Dt, n * 8) || !al(ws.Ut, n * 8) || !al(ws.du, n * 8) ||
         !al(ws.J, colIdx.size() * b * b * vt) || !al(ws.Dinv, (size_t)nNodes * b * b * vt) ||
         !al(ws.vec, (size_t)nvec * n * sizeof(double)) || !al(ws.red, sizeof(double) * kRedBlocks * 80) ||
@@ -1585,7 +1585,7 @@ int nsfv1_block_jacobi(nsfv1_disc* h, const void* vals, int prec, const double* 
     if (!D->hasMesh) { D->fail(NSFV1_ERR_STATE, "block_jacobi: no mesh"); return D->status; }
     if (!vals || !r || !z || (prec != NSFV1_F64 && prec != NSFV1_F32)) { D->fail(NSFV1_ERR_ARGUMENT, "block_jacobi: bad arguments"); return D->status; }
     const int b = D->dim + 1;
-    if (!D->d_bjDinv && !D->cuda_ok(cudaMalloc((void**)&D->d_bjDinv, sizeof(double) * D->nNodes * b * b), "block_jacobi scratch"))
+    if (!D->d_bjDinv && !D->cuda_ok(D->device_malloc((void**)&D->d_bjDinv, sizeof(double) * D->nNodes * b * b), "block_jacobi scratch"))
         return D->status;
     return block_jacobi_run(*D, vals, prec, r, z, D->d_bjDinv, (cudaStream_t)stream) ? NSFV1_OK : D->status;
 }

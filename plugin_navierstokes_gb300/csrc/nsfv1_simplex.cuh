@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(kThreads, DIM == 2 ? (JAC ? 3 : 4) : 2) k_simp
         }
         // ---- upwind (and downwind): velocity, shapes, ncl = |v| / L_up, ndl = |v| / (L_down + L_up)
         double upv[DIM], dnv[DIM], up[NSH], dn[NSH], ncl, ndl = 0.0;
-        const double norm = (upw == UPW_NO || (FLOW && upw == UPW_FULL) || vv < 1.01e-28) ? (vv > 0.0 ? vv * rsqrt(vv) : vv) : 1.0;
+        const double norm = (upw == UPW_NO || (FLOW && upw == UPW_FULL) || vv < 1.01e-28) ? speed(vv) : 1.0;
         if (upw == UPW_FULL) {
             // (sign tests on the bits: a comparison is an FP64 instruction)
             const bool fr = __double_as_longlong(Vn) > 0;                          // upwind corner i, else j
@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(kThreads, DIM == 2 ? (JAC ? 3 : 4) : 2) k_simp
                 // |v| / L = 2 v^2 / sqrt(v^2 l2); the product outside the normal range: one factor at a time
                 const double p = vv * l2;
                 if (p > 1e-280 && p < 1e280) ncl = 2.0 * vv * rsqrt(p);
-                else ncl = vv > 0.0 ? 2.0 * (vv * rsqrt(vv)) * rsqrt(l2) : vv;
+                else ncl = 2.0 * speed(vv) * rsqrt(l2);
             }
         } else if (upw == UPW_LPS && !(norm < 1e-14)) {
             // the ray along -v leaves where the first coordinate N_k - s r_k vanishes

@@ -48,6 +48,12 @@ inline bool plain_params(const DiscParams& P, const bool jac) {
            (P.convUpwind == UPW_NO || P.convUpwind == UPW_FULL || P.convUpwind == UPW_LPS);
 }
 
+// |v| from v^2 in one reciprocal square root; 0, an overflowed square and NaN as the square root has
+// them (the range test on the bits: a comparison is an FP64 instruction)
+__device__ __forceinline__ double speed(const double vv) {
+    return (unsigned long long)(__double_as_longlong(vv) - 1) < 0x7fefffffffffffffULL ? vv * rsqrt(vv) : vv;
+}
+
 template <int DIM, bool SPLIT = false>
 struct Ten {
     static_assert(DIM == 2 || !SPLIT, "a lane per SCVF for quadrilaterals only");
@@ -457,7 +463,7 @@ __global__ void __launch_bounds__(kThreads, DIM == 3 && JAC ? 2 : 3) k_tensor(co
         // ---- upwind (and downwind) velocity, shapes and coefficients: ncl = |v| / L_up,
         // ndl = |v| / (L_down + L_up)
         double upv[DIM], dnv[DIM], up[NSH], dn[NSH], ncl, ndl = 0.0;
-        const double norm = (upw != UPW_LPS || vv < 1.01e-28) ? (vv > 0.0 ? vv * rsqrt(vv) : vv) : 1.0;
+        const double norm = (upw != UPW_LPS || vv < 1.01e-28) ? speed(vv) : 1.0;
         if (upw == UPW_FULL) {
             const bool low = plus ? Vn > 0.0 : !(Vn < 0.0);
 #pragma unroll

@@ -25,6 +25,7 @@
 #include <cuda_bf16.h>
 #include <cudaTypedefs.h>
 #include "nsfv1_gb300.h"
+#include "nsfv1_recip.cuh"
 #include "nsfv1_tc_gemm.cuh"
 
 namespace {
@@ -74,19 +75,7 @@ __device__ __forceinline__ uint64_t mix64(uint64_t z) {
     return z ^ (z >> 31);
 }
 
-// 1 / x for x >= 1: the hardware estimate and one Newton-Raphson step in fused multiply-adds
-// (Markstein, "Computation of elementary functions on the IBM RISC System/6000", 1990).
-// Compared with the IEEE division for every float of [1, 1e37): the same bits; beyond, where
-// |z / x| < 1e-34, within one unit in the last place. Without the division's branch,
-// which kept neighbouring elements of the activation from overlapping.
-__device__ __forceinline__ float recip_ge1(float x) {
-    float r;
-    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
-    const float e = fmaf(-x, r, 1.0f), q = fmaf(r, e, r);
-    return x < 1.0e38f ? q : r;   // x = inf: r = 0
-}
-
-__device__ __forceinline__ float sigmoid(float z) { return recip_ge1(1.0f + expf(-z)); }
+__device__ __forceinline__ float sigmoid(float z) { return nsfv1::recip_ge1(1.0f + expf(-z)); }
 
 // ---- kernels ----------------------------------------------------------------
 

@@ -346,9 +346,17 @@ static cudaError_t launch_fast(int roid, const DiscParams& P, const AsmArgs& a, 
             k_tensor<DIM, JAC, decltype(flow)::value, decltype(affine)::value, SP>
                 <<<grid, t, (size_t)TN::warp_doubles(JAC) * (t / 32) * sizeof(double), s>>>(P, q);
         };
-        // a lane per SCVF while its warps still find a sub-partition each (4 x 152): the launch then takes
-        // one SCVF's chain instead of two (32^2 cells, defect + Jacobian: 143 -> 118 us); with more
-        // elements the shared geometry of a lane's two SCVFs counts more
+        // a lane per SCVF while its warps still find a sub-partition each (4 of 152 SMs): the launch then
+        // takes one SCVF's chain instead of two; with more elements the shared geometry of a lane's two
+        // SCVFs counts more. Four colours, us without -> with the split, defect + Jacobian (and the
+        // defect, the Jacobian alone), FLOW:
+        //   elements of a launch      16            256            2,025          4,830 | 5,625          9,604          22,500
+        //   affine, full upwind       128 -> 106    130 -> 111     132 -> 111     133 -> 118 | 139 -> 129  144 -> 152  265 -> 302
+        //     (defect)                 87 -> 63      87 -> 61       88 -> 62       88 -> 71 |  89 -> 75    99 -> 96   173 -> 177
+        //     (Jacobian)              114 -> 99     112 -> 99      114 -> 100     115 -> 109 | 116 -> 114  126 -> 136  218 -> 276
+        //   general                   139 -> 115    139 -> 115     143 -> 116     142 -> 126 | 143 -> 138  153 -> 167  301 -> 324
+        // LPS as the full upwind. Between the limit and about 7,000 both are within 8 % for the pass that
+        // forms both (the defect alone still gains 16 %), so the line stays at one warp a sub-partition.
         if constexpr (DIM == 2) {
             if (q.count <= 4 * 152 * Ten<2, true>::EPW) { go(std::true_type{}); return; }
         }

@@ -228,7 +228,11 @@ __global__ void __launch_bounds__(256) k_bsr_mv(int64_t nRows, const int32_t* __
 // block is one 128-byte line (with a lane per block, lanes read 128 bytes apart) and a row
 // costs 2 additions per lane for its sums instead of butterflies of four. The FP64 pipe
 // bounds it: 27 multiply-adds and 2 additions per pair of rows at 27 blocks a row.
-// 48^3 hexahedra (3.05 M blocks, 410 MB): 97 us, 4.2 TB/s; 213 us with 8 lanes per row.
+// Trips of nine blocks: an inner row of hexahedra is three of them, one of tetrahedra (about 15
+// blocks) is one and six single blocks. The compiler keeps to 32 registers and starts a trip's
+// loads in groups, not all nine before the first product.
+// 48^3 hexahedra (3.05 M blocks, 410 MB): 97 us, 4.2 TB/s; 213 us with 8 lanes per row. 6 x 40^3
+// tetrahedra 73 -> 39 us, prisms (30^2 x 30) 62 -> 33 us.
 template <int UNROLL>
 __global__ void __launch_bounds__(256) k_bsr_mv_f64x4(int64_t nRows, const int32_t* __restrict__ rowPtr, const int32_t* __restrict__ colIdx,
                                                       const double* __restrict__ vals, const double* __restrict__ x, double* __restrict__ y,
@@ -241,7 +245,6 @@ __global__ void __launch_bounds__(256) k_bsr_mv_f64x4(int64_t nRows, const int32
     double acc = 0.0;
     int q = q0;
     for (; q + UNROLL <= q1; q += UNROLL) {
-        // the loads of UNROLL blocks are issued before the first product
         double a[UNROLL], xv[UNROLL];
         int c[UNROLL];
 #pragma unroll
@@ -688,7 +691,7 @@ __global__ void k_set_dirichlet(int64_t n, const int32_t* __restrict__ rows, con
 // Four FP64 multiply-adds per basis entry on a pipe that takes a warp instruction
 // every 19 clocks per SM (about 14 us an iteration at 192^2 quadrilaterals, n =
 // 111,747, 16 basis vectors) and the L2 round trips of the reductions bound it:
-// 68 us an iteration there (GMRES(30), 45 iterations in 3.04 ms; 64^2: 44 us). With
+// 67 us an iteration there (GMRES(30), 45 iterations in 3.00 ms; 64^2: 43 us). With
 // one dot product per pass over w, a single-block sum of every coefficient and three
 // host reads an iteration it was 214 us (9.64 ms; 64^2: 200 us). Launching the five
 // kernels with programmatic stream serialisation measured the same (3.12 ms).

@@ -259,7 +259,8 @@ __global__ void __launch_bounds__(128, 1)
 // The activation's instructions bound it: a tile's MMAs take 1.2 us. Measured at K = 256:
 // 81 us for 249,728 rows; with 16-byte stores straight from the lanes 121 us. 532,512 points
 // through all layers and the head: 0.95 ms, 3.13 ms when the FP32 product went through memory to
-// an activation kernel that also wrote a transposed copy.
+// an activation kernel that also wrote a transposed copy. 96 registers a thread (576 threads); the
+// training variant (ACT and STORE_A) spills 40 bytes, the others nothing.
 // ---------------------------------------------------------------------------
 template <int K>
 struct LayerSmem {

@@ -27,7 +27,7 @@
 //  * the Jacobian blocks of a warp pass through shared memory and are reduced into the
 //    matrix by consecutive entries.
 // Counted per hexahedron: 7.7 k FP64 instructions for LPS + FLOW defect and Jacobian (13.2 k
-// before), with the FP64 pipe 78 % active (its practical limit is 16/19). Measured, one thread
+// before), with the FP64 pipe 77 % active (its practical limit is 16/19). Measured, one thread
 // per element before -> here: 64^3 affine, defect + Jacobian 7.73 -> 4.47 ms; 41^3 distorted
 // transient, defect 2.56 -> 0.92 ms; 32^2 quadrilaterals 293 -> 118 us (143 without SPLIT). With 8-byte reductions
 // straight from the lanes the first was 5.6 ms (138 G sectors/s into L2).

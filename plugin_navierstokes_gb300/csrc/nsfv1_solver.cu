@@ -978,8 +978,9 @@ __global__ void __launch_bounds__(kGmT) k_gm_end(int64_t n, int j, const double*
 // the scalar end of iteration j (one block): the Hessenberg column h1 + h2, the Givens
 // rotations, the residual estimate and the stop tests. The rotations are one serial chain of
 // FP64 operations (64 clocks each): its inputs come to shared memory first.
-// The host follows in pinned memory: the iteration count, and at a stop the state, then G_DONE.
-__device__ __forceinline__ void gm_givens(double* G, volatile double* host, const int j, const int m, const double rtol) {
+// The host follows in pinned memory: the iteration count (one write, since the host keeps reading the
+// line), and at a stop or the end of a cycle ('last') the state, then G_DONE.
+__device__ __forceinline__ void gm_givens(double* G, volatile double* host, const int j, const int m, const double rtol, const bool last) {
     __shared__ double hc[kGmMaxM + 1], cs[kGmMaxM], sn[kGmMaxM];
     const int t = threadIdx.x;
     if (t <= j) hc[t] = G[G_H1 + t] + G[G_H2 + t];
@@ -1004,9 +1005,11 @@ __device__ __forceinline__ void gm_givens(double* G, volatile double* host, cons
         G[G_RELRES] = relres;
         G[G_IT] = it + 1.0;
         const int done = !isfinite(relres) ? GM_NONFINITE : relres < rtol || hn == 0.0 ? GM_CYCLE_END : 0;
-        host[G_RELRES] = relres;
-        host[G_J] = j + 1;
         host[G_IT] = it + 1.0;
+        if (done || last) {
+            host[G_RELRES] = relres;
+            host[G_J] = j + 1;
+        }
         if (done) {
             G[G_DONE] = done;
             __threadfence_system();
@@ -1018,7 +1021,7 @@ __device__ __forceinline__ void gm_givens(double* G, volatile double* host, cons
 }
 
 __global__ void __launch_bounds__(kGmT) k_gm_givens(double* G, double* host, int j, int m, double rtol) {
-    if (G[G_DONE] == 0.0) gm_givens(G, host, j, m, rtol);
+    if (G[G_DONE] == 0.0) gm_givens(G, host, j, m, rtol, true);
 }
 
 // V_j *= 1 / norm; Z_j = Dinv V_j (the point-block Jacobi apply of k_prec, same summation).
@@ -1029,7 +1032,7 @@ template <typename MT, int b>
 __global__ void __launch_bounds__(kGmT) k_gm_prec(int64_t nRows, double* G, double* host, double* __restrict__ Vj,
                                                   const MT* __restrict__ Dinv, double* __restrict__ Zj, int j, int m, double rtol) {
     if (blockIdx.x == gridDim.x - 1) {
-        if (j > 0 && G[G_DONE] == 0.0) gm_givens(G, host, j - 1, m, rtol);
+        if (j > 0 && G[G_DONE] == 0.0) gm_givens(G, host, j - 1, m, rtol, false);
         return;
     }
     const int64_t r = (int64_t)blockIdx.x * kGmT + threadIdx.x;
@@ -1307,11 +1310,14 @@ static constexpr int kGmresAhead = 3;
 
 // waits until the device has ended 'iters' iterations, has stopped, or has nothing queued any more
 static bool gmres_wait(Disc& D, const volatile double* host, int iters, cudaStream_t s) {
+    if (!D.cuda_ok(cudaGetLastError(), "gmres launch")) return false;
     for (int spin = 1; host[G_IT] < iters && host[G_DONE] == 0.0; ++spin) {
-        if (spin % 256) continue;
+        for (volatile int k = 0; k < 200; ++k) {}   // a read about every 0.2 us
+        if (spin % 64) continue;
         const cudaError_t e = cudaStreamQuery(s);
         if (e == cudaSuccess) break;
         if (e != cudaErrorNotReady) return D.cuda_ok(e, "gmres state");
+        cudaGetLastError();   // "not ready" is no error of a launch
     }
     return true;
 }
